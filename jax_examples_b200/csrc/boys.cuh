@@ -185,6 +185,97 @@ __device__ __forceinline__ void boys_eval(T t, const T* __restrict__ tabA, T (&F
   }
 }
 
+// 1 / sqrt(x) for normal positive x: the hardware's approximation refined by
+// one third-order Householder step, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2
+// (the next term is 5 e^3/16).  Against rsqrt() it spares the range checks and
+// their branch.
+__device__ __forceinline__ double rsqrt_refined(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ float rsqrt_refined(float x) { return rsqrtf(x); }
+
+// Where boys_hermite leaves the table: above this T the terms in e^{-T} of the
+// upward recursion are below 2^-60 of every F_m, m <= M (below 2^-30 in FP32;
+// F_0 has none, and differs from sqrt(pi/T)/2 by erfc(6) = 2e-17 at 36).
+template <typename T>
+__host__ __device__ constexpr int boys_far(int M) {
+  return sizeof(T) == 4 || M == 0 ? int(kBoysTMax) : boys_exp_tcut(M);
+}
+
+// Rn[n] = W (p+q)^{-1/2} (-2 rho)^n F_n(rho R2), n = 0 .. M, rho = pq/(p+q):
+// the Hermite recursion's start values, without forming F_n where it is not
+// needed.  With u = pq R2 the argument is T = u/(p+q), so the side of the
+// table's end is known before any root is taken, and one root serves both
+// sides: of p+q in the table (T = u y^2, rho = pq y^2), of u beyond it, where
+//   (p+q)^{-1/2} F_0 = sqrt(pi)/2 u^{-1/2}   and   -2 rho F_{n+1}/F_n = -(2n+1)/R2
+// with 1/R2 = pq y^2: no table access, no exponential, n multiplications.
+// The two-sided form (a root of p+q, then one of T on one side) took about 75
+// instructions a lane and s-type primitive quartet in a diverged warp; warp
+// instructions of a (H2O)16 full build: (ss|ss) 290 -> 234 M, (ps|ss) 517 ->
+// 366 M, whole build 7.17 -> 6.76 ms serial.
+template <typename T, int M>
+__device__ __forceinline__ void boys_hermite(T pq, T s, T R2, T W, const T* __restrict__ tabA, T (&Rn)[M + 1]) {
+  static_assert(boys_far<T>(M) <= kBoysTabT, "Boys table too short");
+  constexpr int KT = BoysConst<T>::kTaylor;
+  constexpr bool kDeriv = M > 0 && M <= kBoysDerivMaxM;
+  constexpr int KP = (kDeriv && KT < kBoysARow) ? KT + 1 : KT;
+  const T u = pq * R2;
+  const bool near = u < T(boys_far<T>(M)) * s;
+  const T x = near ? s : u;
+  const T y = rsqrt_refined(x);
+  // 1/x by one Newton step on y^2: its powers below would multiply y's rounding
+  T inv = y * y;
+  inv = fma(inv, fma(-x, inv, T(1)), inv);
+  const T g = pq * inv;  // rho in the table, 1/R2 beyond
+  T pref = W * y;
+  if (near) {
+    const T t = R2 * g;
+    const T xr = t * T(kBoysGridInv) + RoundMagic<T>::value;
+    const int i = RoundMagic<T>::low(xr);
+    const T d = (xr - RoundMagic<T>::value) * T(1.0 / kBoysGridInv) - t;  // T_i - t, |d| <= 1/32
+    T v[8];
+    boys_row(tabA + (M * kBoysRows + i) * kBoysARow, v);
+    T F = v[KP - 1], e = T(0);
+    if constexpr (kDeriv) {
+      T der = T(0);
+#pragma unroll
+      for (int k = KP - 2; k >= 0; --k) {
+        der = der * d + F;
+        F = F * d + v[k];
+      }
+      e = T(2 * M + 1) * F - (t + t) * der;
+    } else {
+#pragma unroll
+      for (int k = KT - 2; k >= 0; --k) F = F * d + v[k];
+      if constexpr (M > 0) {
+        T ed = T(inv_factorial(KT - 1));
+#pragma unroll
+        for (int k = KT - 2; k >= 0; --k) ed = ed * d + T(inv_factorial(k));
+        e = __ldg(tabA + kBoysExpOff + i) * ed;
+      }
+    }
+    Rn[M] = F;
+    if constexpr (M > 0) {
+      const T t2 = t + t;
+#pragma unroll
+      for (int m = M - 1; m >= 0; --m) Rn[m] = (t2 * Rn[m + 1] + e) * T(1.0 / (2 * m + 1));
+    }
+    const T m2rho = T(-2) * g;
+#pragma unroll
+    for (int m = 0; m <= M; ++m) {
+      Rn[m] *= pref;
+      if (m < M) pref *= m2rho;
+    }
+  } else {
+    Rn[0] = T(0.88622692545275801364908374167057) * pref;  // sqrt(pi)/2
+#pragma unroll
+    for (int m = 0; m < M; ++m) Rn[m + 1] = Rn[m] * (T(-(2 * m + 1)) * g);
+  }
+}
+
 // Runtime-order variant for the standalone Boys kernel (m <= kBoysMaxM).
 template <typename T>
 __device__ __forceinline__ void boys_eval_rt(T t, const T* __restrict__ tab, int M, T* F) {

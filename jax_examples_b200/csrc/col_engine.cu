@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(32 * kColWarps) col_jk_kernel(const JKParams p
     const int p0 = task.flags & 0xffff, p1 = task.flags >> 16;
     col_quartet<T, LA, LB, LC, LD>(sm, pp + bp.pp + p0, p1 - p0, A, B, pp + kp.pp, kp.npp, C, Dv, tab, lane);
     double s = 1.0;
-    if (bp.diag) s *= 0.5;
-    if (kp.diag) s *= 0.5;
+    if (bp.diag()) s *= 0.5;
+    if (kp.diag()) s *= 0.5;
     if (task.bra == kidx) s *= 0.5;
     warp_digest_jk<T>(prm, sm->blk, ncart(LA), ncart(LB), ncart(LC), ncart(LD), prm.ao[bp.a], prm.ao[bp.b],
                       prm.ao[kp.a], prm.ao[kp.b], s, lane);

@@ -276,6 +276,8 @@ struct jqc_ctx {
   DevBuf<ShellPair> d_pairs;
   DevBuf<PrimPair> d_pp;
   DevBuf<PrimPairF> d_ppf;
+  DevBuf<PrimRec> d_rec;   // the same pairs as compact records, primitive-major inside a block
+  DevBuf<PrimRecF> d_recf;
   // work lists: one per (precision mode, mixed_tau) in use, plus the dense one
   std::vector<TaskSet*> jk_cache;
   TaskSet* jk_cur = nullptr;
@@ -741,6 +743,7 @@ static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D
       if (p.n_tasks == 0) continue;
       p.pairs = c->d_pairs.ptr;
       p.pp = prec ? (const void*)c->d_ppf.ptr : (const void*)c->d_pp.ptr;
+      p.rec = prec ? (const void*)c->d_recf.ptr : (const void*)c->d_rec.ptr;
       p.centres = c->d_centres.ptr;
       p.ao = c->d_ao.ptr;
       p.boys = prec ? (const void*)c->boys32 : (const void*)c->boys64;
@@ -1034,19 +1037,22 @@ int jqc_pairs_build(jqc_ctx* c, double schwarz_tau, double prim_tau, void* strea
       make_prim_pairs(c, a, b, rawpp);
       sp.npp = (int)rawpp.size() - sp.pp;
       sp.Q = 0.0;
-      sp.diag = (a == b);
-      sp.cls = pair_class(c->l[a], c->l[b]);
-      ids[sp.cls].push_back((int)raw.size());
+      sp.rec = sp.pp;  // one pair after the other until the pairs are sorted into blocks
+      sp.stride_diag = (1u << 1) | unsigned(a == b);
+      ids[pair_class(c->l[a], c->l[b])].push_back((int)raw.size());
       raw.push_back(sp);
     }
   c->n_pairs_all = (long long)raw.size();
   // 2. Schwarz bounds on the device
   DevBuf<ShellPair> d_raw;
   DevBuf<PrimPair> d_rawpp;
+  DevBuf<PrimRec> d_rawrec;
   DevBuf<unsigned long long> d_q;
   DevBuf<int> d_ids;
   JQC_CUDA_CHECK(d_raw.upload(raw, s));
   JQC_CUDA_CHECK(d_rawpp.upload(rawpp, s));
+  JQC_CUDA_CHECK(d_rawrec.reserve(rawpp.size()));
+  JQC_CUDA_CHECK(launch_prim_rec(d_raw.ptr, (int)raw.size(), d_rawpp.ptr, d_rawrec.ptr, nullptr, s));
   JQC_CUDA_CHECK(d_q.reserve(raw.size()));
   JQC_CUDA_CHECK(cudaMemsetAsync(d_q.ptr, 0, raw.size() * sizeof(unsigned long long), s));
   std::vector<int> all_ids;
@@ -1062,6 +1068,7 @@ int jqc_pairs_build(jqc_ctx* c, double schwarz_tau, double prim_tau, void* strea
     p.n_pairs = (int)ids[pc].size();
     p.pairs = d_raw.ptr;
     p.pp = d_rawpp.ptr;
+    p.rec = d_rawrec.ptr;
     p.centres = c->d_centres.ptr;
     p.boys = c->boys64;
     p.boys_al = c->boysA64;
@@ -1090,7 +1097,7 @@ int jqc_pairs_build(jqc_ctx* c, double schwarz_tau, double prim_tau, void* strea
     if (raw[k].Q * qmax[c->shell_mol[raw[k].a]] >= schwarz_tau && raw[k].Q > 0.0) keep.push_back((int)k);
   auto key = [&](int k) {
     const ShellPair& p = raw[k];
-    return std::make_tuple(p.cls, p.npp, c->shell_mol[p.a]);
+    return std::make_tuple(pair_class(c->l[p.a], c->l[p.b]), p.npp, c->shell_mol[p.a]);
   };
   std::stable_sort(keep.begin(), keep.end(), [&](int x, int y) {
     auto kx = key(x), ky = key(y);
@@ -1119,9 +1126,20 @@ int jqc_pairs_build(jqc_ctx* c, double schwarz_tau, double prim_tau, void* strea
     c->blocks.back().count++;
     c->pairs.push_back(sp);
   }
+  // compact records: record i of the block's k-th pair at (first of the block)
+  // + i * count + k
+  for (const Block& B : c->blocks)
+    for (int k = 0; k < B.count; ++k) {
+      ShellPair& sp = c->pairs[B.start + k];
+      sp.rec = c->pairs[B.start].pp + k;
+      sp.stride_diag = (unsigned(B.count) << 1) | unsigned(sp.diag());
+    }
   JQC_CUDA_CHECK(c->d_pairs.upload(c->pairs, s));
   JQC_CUDA_CHECK(c->d_pp.upload(pp, s));
   JQC_CUDA_CHECK(c->d_ppf.upload(ppf, s));
+  JQC_CUDA_CHECK(c->d_rec.reserve(pp.size()));
+  JQC_CUDA_CHECK(c->d_recf.reserve(pp.size()));
+  JQC_CUDA_CHECK(launch_prim_rec(c->d_pairs.ptr, (int)c->pairs.size(), c->d_pp.ptr, c->d_rec.ptr, c->d_recf.ptr, s));
   JQC_CUDA_CHECK(cudaStreamSynchronize(s));
   c->tau = schwarz_tau;
   c->pairs_ready = true;
@@ -1251,6 +1269,7 @@ int jqc_eri_tensor(jqc_ctx* c, double* out, long long max_bytes, void* stream) {
     p.n_tasks = c->full_tasks.cnt[0][qc];
     p.pairs = c->d_pairs.ptr;
     p.pp = c->d_pp.ptr;
+    p.rec = c->d_rec.ptr;
     p.centres = c->d_centres.ptr;
     p.ao = c->d_ao.ptr;
     p.boys = c->boys64;

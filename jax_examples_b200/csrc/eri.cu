@@ -24,12 +24,12 @@ struct SchwarzBody {
     const int id = prm.pair_ids[pid];
     const ShellPair bp = prm.pairs[id];
     const double* ctr = prm.centres;
-    Vec3<double> A{ctr[3 * bp.a], ctr[3 * bp.a + 1], ctr[3 * bp.a + 2]};
-    Vec3<double> B{ctr[3 * bp.b], ctr[3 * bp.b + 1], ctr[3 * bp.b + 2]};
+    const double *A = ctr + 3 * bp.a, *B = ctr + 3 * bp.b;
     double out[Cfg::NAB][Cfg::CDP];
     double ebuf[3][LA + 1][LB + 1][LA + LB + 1];
-    quartet_accumulate<double, LA, LB, LA, LB, NS, PART, false>(prm.pp + bp.pp, bp.npp, A, B, prm.pp + bp.pp,
-                                                                 bp.npp, A, B, prm.boys_al, ebuf, out);
+    const PrimList<double, true> prims{prm.rec + bp.rec, bp.stride(), bp.npp};
+    quartet_accumulate<double, LA, LB, LA, LB, NS, PART, false>(prims, prims, quartet_geom<double>(A, B, A, B),
+                                                                 prm.boys_al, ebuf, out);
     double m = 0.0;
     static_for<Cfg::NCDP>([&](auto c_) {
       constexpr int cdi = decltype(c_)::value;
@@ -95,24 +95,21 @@ struct PrimBody {
     using Cfg = QCfg<LA, LB, LC, LD, NS, PART>;
     const double* ex = prm.exps + 4 * q;
     const double* c = prm.centres + 12 * q;
-    Vec3<double> A{c[0], c[1], c[2]}, B{c[3], c[4], c[5]}, C{c[6], c[7], c[8]}, D{c[9], c[10], c[11]};
-    PrimPair bra, ket;
-    {
-      const double al = ex[0], be = ex[1], p = al + be;
-      const double dx = A.x - B.x, dy = A.y - B.y, dz = A.z - B.z;
-      bra = PrimPair{p, 0.5 / p, (al * A.x + be * B.x) / p, (al * A.y + be * B.y) / p, (al * A.z + be * B.z) / p,
-                     exp(-(al * be / p) * (dx * dx + dy * dy + dz * dz)), al, be};
-    }
-    {
-      const double al = ex[2], be = ex[3], p = al + be;
-      const double dx = C.x - D.x, dy = C.y - D.y, dz = C.z - D.z;
-      ket = PrimPair{p, 0.5 / p, (al * C.x + be * D.x) / p, (al * C.y + be * D.y) / p, (al * C.z + be * D.z) / p,
-                     exp(-(al * be / p) * (dx * dx + dy * dy + dz * dz)), al, be};
-    }
+    const QuartetGeom<double> geo = quartet_geom<double>(c, c + 3, c + 6, c + 9);
+    auto make = [](double al, double be, const Vec3<double>& d) {
+      // one reciprocal; the two quotients take Markstein's residual correction
+      const double p = al + be, inv = 1.0 / p, ab = al * be;
+      double x = ab * inv, t = be * inv;
+      x = fma(fma(-x, p, ab), inv, x);
+      t = fma(fma(-t, p, be), inv, t);
+      const double h = 0.5 * inv, K = exp(-x * (d.x * d.x + d.y * d.y + d.z * d.z));
+      return PrimRec{p, t, K * h * kSqrt8Pi25, h};
+    };
+    const PrimRec bra = make(ex[0], ex[1], geo.AB), ket = make(ex[2], ex[3], geo.CD);
     double out[Cfg::NAB][Cfg::CDP];
     double ebuf[3][LA + 1][LB + 1][LA + LB + 1];
-    quartet_accumulate<double, LA, LB, LC, LD, NS, PART, false, false>(&bra, 1, A, B, &ket, 1, C, D, prm.boys_al,
-                                                                        ebuf, out);
+    quartet_accumulate<double, LA, LB, LC, LD, NS, PART, false, false>(
+        PrimList<double, false>{&bra, 1, 1}, PrimList<double, false>{&ket, 1, 1}, geo, prm.boys_al, ebuf, out);
     static_for<Cfg::NAB * Cfg::NCDP>([&](auto x_) {
       constexpr int x = decltype(x_)::value;
       constexpr int ab = x / Cfg::NCDP, cdi = x % Cfg::NCDP;
@@ -346,6 +343,30 @@ cudaError_t launch_symmetrize(double* M, int count, int n, cudaStream_t s) {
   const long long tot = (long long)n * n * count;
   if (tot == 0) return cudaSuccess;
   symmetrize_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(M, count, n);
+  return cudaGetLastError();
+}
+
+// Compact records of the primitive pairs (and their FP32 copies, unless recf is
+// null), one thread a pair: record i of a pair at rec + i * stride().
+__global__ void __launch_bounds__(128) prim_rec_kernel(const ShellPair* __restrict__ pairs, int n_pairs,
+                                                       const PrimPair* __restrict__ pp, PrimRec* __restrict__ rec,
+                                                       PrimRecF* __restrict__ recf) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n_pairs) return;
+  const ShellPair sp = pairs[k];
+  for (int i = 0; i < sp.npp; ++i) {
+    const PrimPair q = ld_pp(pp + sp.pp + i);
+    const PrimRec r{q.p, q.beta / q.p, q.K * q.h * kSqrt8Pi25, q.h};
+    const long long at = sp.rec + (long long)i * sp.stride();
+    rec[at] = r;
+    if (recf != nullptr) recf[at] = PrimRecF{float(r.p), float(r.t), float(r.W), float(r.h)};
+  }
+}
+
+cudaError_t launch_prim_rec(const ShellPair* pairs, int n_pairs, const PrimPair* pp, PrimRec* rec, PrimRecF* recf,
+                            cudaStream_t s) {
+  if (n_pairs == 0) return cudaSuccess;
+  prim_rec_kernel<<<unsigned((n_pairs + 127) / 128), 128, 0, s>>>(pairs, n_pairs, pp, rec, recf);
   return cudaGetLastError();
 }
 

@@ -27,13 +27,12 @@ struct TensorBody {
     const ShellPair bp = prm.pairs[task.bra];
     const ShellPair kp = prm.pairs[task.ket0 + (active ? lane : 0)];
     const double* ctr = prm.centres;
-    Vec3<double> A{ctr[3 * bp.a], ctr[3 * bp.a + 1], ctr[3 * bp.a + 2]};
-    Vec3<double> B{ctr[3 * bp.b], ctr[3 * bp.b + 1], ctr[3 * bp.b + 2]};
-    Vec3<double> C{ctr[3 * kp.a], ctr[3 * kp.a + 1], ctr[3 * kp.a + 2]};
-    Vec3<double> D{ctr[3 * kp.b], ctr[3 * kp.b + 1], ctr[3 * kp.b + 2]};
+    const QuartetGeom<double> geo =
+        quartet_geom<double>(ctr + 3 * bp.a, ctr + 3 * bp.b, ctr + 3 * kp.a, ctr + 3 * kp.b);
     double out[Cfg::NAB][Cfg::CDP];
-    quartet_accumulate<double, LA, LB, LC, LD, NS, PART, true>(prm.pp + bp.pp, bp.npp, A, B, prm.pp + kp.pp,
-                                                                active ? kp.npp : 0, C, D, prm.boys_al, ebra, out);
+    quartet_accumulate<double, LA, LB, LC, LD, NS, PART, true>(
+        PrimList<double, true>{prm.rec + bp.rec, bp.stride(), bp.npp},
+        PrimList<double, true>{prm.rec + kp.rec, kp.stride(), active ? kp.npp : 0}, geo, prm.boys_al, ebra, out);
     if (!active) return;
     const long long n = prm.n;
     const long long a0 = prm.ao[bp.a], b0 = prm.ao[bp.b], c0 = prm.ao[kp.a], d0 = prm.ao[kp.b];

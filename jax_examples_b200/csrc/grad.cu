@@ -334,8 +334,8 @@ __global__ void __launch_bounds__(32 * kGradWarps, 4) warp_grad_kernel(const Gra
     }
     // reduce over the warp and scatter to the four atoms
     double sc = 4.0;
-    if (bp.diag) sc *= 0.5;
-    if (kp.diag) sc *= 0.5;
+    if (bp.diag()) sc *= 0.5;
+    if (kp.diag()) sc *= 0.5;
     if (task.bra == kidx) sc *= 0.5;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {

@@ -278,8 +278,8 @@ struct GradBody {
     }
     // scatter: 4 s per canonical quartet; bra centres reduced over the warp
     double sc = active ? 4.0 : 0.0;
-    if (bp.diag) sc *= 0.5;
-    if (kp.diag) sc *= 0.5;
+    if (bp.diag()) sc *= 0.5;
+    if (kp.diag()) sc *= 0.5;
     if (task.bra == kidx) sc *= 0.5;
     static_for<9>([&](auto k) { g[decltype(k)::value] *= sc; });
     double* pf = prm.pair_force;
@@ -349,21 +349,27 @@ cudaError_t launch_grad_class(const GradParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Classes whose gradient runs in the register kernels.
-#define JQC_FOR_GRAD_REG_CLASSES(X) \
-  X(0, 0, 0, 0, 0)                  \
-  X(1, 1, 0, 0, 0)                  \
-  X(2, 1, 0, 1, 0)                  \
-  X(3, 1, 1, 0, 0)                  \
-  X(4, 1, 1, 1, 0)                  \
-  X(6, 2, 0, 0, 0)                  \
-  X(7, 2, 0, 1, 0)                  \
-  X(10, 2, 1, 0, 0)                 \
-  X(5, 1, 1, 1, 1)                  \
-  X(8, 2, 0, 1, 1)                  \
-  X(9, 2, 0, 2, 0)                  \
-  X(11, 2, 1, 1, 0)                 \
-  X(15, 2, 2, 0, 0)
-
+// Classes whose gradient runs in the register kernels, by compilation unit
+// (the unrolled classes take minutes each to compile).
+#define JQC_FOR_GRAD_REG_SP(X) \
+  X(0, 0, 0, 0, 0)             \
+  X(1, 1, 0, 0, 0)             \
+  X(2, 1, 0, 1, 0)             \
+  X(3, 1, 1, 0, 0)             \
+  X(4, 1, 1, 1, 0)             \
+  X(5, 1, 1, 1, 1)
+#define JQC_FOR_GRAD_REG_DS(X) \
+  X(6, 2, 0, 0, 0)             \
+  X(7, 2, 0, 1, 0)             \
+  X(8, 2, 0, 1, 1)             \
+  X(9, 2, 0, 2, 0)
+#define JQC_FOR_GRAD_REG_DP(X) \
+  X(10, 2, 1, 0, 0)            \
+  X(11, 2, 1, 1, 0)
+#define JQC_FOR_GRAD_REG_DD(X) X(15, 2, 2, 0, 0)
+cudaError_t launch_grad_reg_sp(int qc, const GradParams& p, cudaStream_t s);
+cudaError_t launch_grad_reg_ds(int qc, const GradParams& p, cudaStream_t s);
+cudaError_t launch_grad_reg_dp(int qc, const GradParams& p, cudaStream_t s);
+cudaError_t launch_grad_reg_dd(int qc, const GradParams& p, cudaStream_t s);
 
 }  // namespace jqc

@@ -373,8 +373,8 @@ __global__ void __launch_bounds__(32 * kGRowWarps, grad_row_min_blocks(LA, LB, L
     }
     // reduce over the warp and add to the shell-pair force slots
     double sc = 4.0;
-    if (bp.diag) sc *= 0.5;
-    if (kp.diag) sc *= 0.5;
+    if (bp.diag()) sc *= 0.5;
+    if (kp.diag()) sc *= 0.5;
     if (task.bra == kidx) sc *= 0.5;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {

@@ -49,7 +49,6 @@ struct JKBody {
   template <int PART>
   __device__ __forceinline__ void body() {
     using Cfg = QCfg<LA, LB, LC, LD, NS, PART>;
-    using PPT = typename PPType<T>::type;
     constexpr int NA = Cfg::NA, NB = Cfg::NB, ND = Cfg::ND;
     constexpr int NCDP = Cfg::NCDP;
 
@@ -102,22 +101,21 @@ struct JKBody {
     }
     if (__ballot_sync(0xffffffffu, active) == 0u) return;
 
-    const PPT* pp = static_cast<const PPT*>(prm.pp);
+    using Rec = typename RecType<T>::type;
+    const Rec* rec = static_cast<const Rec*>(prm.rec);
     const double* ctr = prm.centres;
-    Vec3<T> A{T(ctr[3 * bp.a]), T(ctr[3 * bp.a + 1]), T(ctr[3 * bp.a + 2])};
-    Vec3<T> B{T(ctr[3 * bp.b]), T(ctr[3 * bp.b + 1]), T(ctr[3 * bp.b + 2])};
-    Vec3<T> C{T(ctr[3 * kp.a]), T(ctr[3 * kp.a + 1]), T(ctr[3 * kp.a + 2])};
-    Vec3<T> D{T(ctr[3 * kp.b]), T(ctr[3 * kp.b + 1]), T(ctr[3 * kp.b + 2])};
+    const QuartetGeom<T> geo = quartet_geom<T>(ctr + 3 * bp.a, ctr + 3 * bp.b, ctr + 3 * kp.a, ctr + 3 * kp.b);
 
     T out[Cfg::NAB][Cfg::CDP];
     const int p0 = task.flags & 0xffff, p1 = task.flags >> 16;  // bra primitive-pair range
-    quartet_accumulate<T, LA, LB, LC, LD, NS, PART, true>(pp + bp.pp + p0, p1 - p0, A, B, pp + kp.pp,
-                                                           active ? kp.npp : 0, C, D, static_cast<const T*>(prm.boys_al),
-                                                           ebra, out);
+    quartet_accumulate<T, LA, LB, LC, LD, NS, PART, true>(
+        PrimList<T, true>{rec + bp.rec + (long long)p0 * bp.stride(), bp.stride(), p1 - p0},
+        PrimList<T, true>{rec + kp.rec, kp.stride(), active ? kp.npp : 0}, geo, static_cast<const T*>(prm.boys_al),
+        ebra, out);
 
     double s = active ? 1.0 : 0.0;
-    if (bp.diag) s *= 0.5;
-    if (kp.diag) s *= 0.5;
+    if (bp.diag()) s *= 0.5;
+    if (kp.diag()) s *= 0.5;
     if (task.bra == kidx) s *= 0.5;
 
     // Segmented suffix sums over lanes of one task (packed warps): bit k of
@@ -303,8 +301,23 @@ struct JKBody {
 // Warps walk the task list with a grid stride: one task per warp when the
 // grid covers the list, several (a persistent grid of resident blocks) when
 // the launch caps the grid.
+// Registers a thread may use.  The FP64 classes of low L wait on loads and on
+// FP64 results, and a few more resident warps are worth a few spilled values;
+// the larger ones lose more to the spills.  (H2O)16 full build, each class by
+// itself, us: (ps|ss) 98 -> 80 registers 942 -> 860 (72: 862, 96: 857, 128:
+// 905), (pp|ss) 138 -> 128 243 -> 225 (96: 235, 168: 246), (ds|ps) 180 -> 168
+// 614 -> 532 (96: 661, 128: 538), (dp|ss) 210 -> 128 385 -> 320 (96: 386, 168:
+// 337); every other class was slowest at the ends of 64 .. 168 and fastest at
+// the value here or unrestricted, and the FP32 classes did not care.
+template <typename T>
+__host__ __device__ constexpr int jk_register_cap(int la, int lb, int lc, int ld) {
+  const int qc = quartet_class(pair_class(la, lb), pair_class(lc, ld));
+  if (sizeof(T) == 4) return qc == 0 ? 72 : qc == 1 ? 96 : 255;
+  return qc <= 1 ? 80 : (qc == 2 || qc == 3 || qc == 6 || qc == 10) ? 128 : qc == 7 ? 168 : 255;
+}
+
 template <typename T, int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(kMaxJKThreads) jk_kernel(const JKParams prm) {
+__global__ void __maxnreg__(jk_register_cap<T>(LA, LB, LC, LD)) jk_kernel(const JKParams prm) {
   constexpr int NS = class_split(LA, LB, LC, LD);
   __shared__ T sE[kMaxJKThreads / 32][3][LA + 1][LB + 1][LA + LB + 1];
   const int stride = int((gridDim.x * blockDim.x) >> 5);

@@ -23,6 +23,7 @@ struct JKParams {
   int n_tasks;
   const ShellPair* pairs;
   const void* pp;          // PrimPair* (FP64) or PrimPairF* (FP32)
+  const void* rec;         // PrimRec* (FP64) or PrimRecF* (FP32)
   const double* centres;   // 3 per shell
   const int* ao;           // first basis function of each shell
   const void* boys;        // Boys table of the kernel's type (row-major)
@@ -80,6 +81,7 @@ struct TensorParams {
   int n_tasks;
   const ShellPair* pairs;
   const PrimPair* pp;
+  const PrimRec* rec;
   const double* centres;
   const int* ao;
   const double* boys;
@@ -93,6 +95,7 @@ struct SchwarzParams {
   int n_pairs;
   const ShellPair* pairs;
   const PrimPair* pp;
+  const PrimRec* rec;
   const double* centres;
   const double* boys;
   const double* boys_al;
@@ -120,6 +123,10 @@ cudaError_t launch_boys(const double* T, long long n, int mmax, void* out, bool 
 cudaError_t launch_dmax(const double* D, int n_dens, int n, int n_shell, const int* ao, const int* l, float* dmax,
                         float* dmax_top, cudaStream_t s);
 cudaError_t launch_symmetrize(double* M, int count, int n, cudaStream_t s);
+// The compact records (recf: may be null) of n_pairs shell pairs from their
+// primitive pairs.
+cudaError_t launch_prim_rec(const ShellPair* pairs, int n_pairs, const PrimPair* pp, PrimRec* rec, PrimRecF* recf,
+                            cudaStream_t s);
 // Writes, for every segment, the indices of the work items that survive into
 // segs[k].out and their count into *segs[k].count (the counts must be zero on
 // entry).  An item survives when (with mol_active) one of its tasks belongs to

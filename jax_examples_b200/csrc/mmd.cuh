@@ -55,12 +55,56 @@ struct PPType<float> {
   using type = PrimPairF;
 };
 
-// Shell pair (a, b) with la >= lb.  pp/npp index its primitive pairs.
+// The same primitive pair as the register kernels read it: everything relative
+// to the shell pair's own centres.  t = beta / p, so P - A = t (B - A) and
+// P - B = (P - A) - (B - A); W = K h sqrt(8 pi^{5/2}), so the prefactor of a
+// primitive quartet is W_ab W_cd / sqrt(p + q).  A lane's load writes its full
+// width back to the registers whether or not the address is shared (128 bytes
+// a cycle and SM), and that data path, 80% busy, bound the low-L kernels: 32
+// bytes a primitive pair instead of 64 is what this record is for ((H2O)16 full
+// build: (ss|ss) 595 -> 550 us, (ds|ss) 522 -> 494, (ps|ps) 449 -> 430; the
+// closed-form tail of boys_hermite took them to 522, 474, 421).  Distances
+// formed from differences of centres are also no less accurate than those of
+// absolute positions (in FP32 markedly more).
+struct __align__(32) PrimRec {
+  double p, t, W, h;
+};
+struct __align__(16) PrimRecF {
+  float p, t, W, h;
+};
+static_assert(sizeof(PrimRec) == 32 && sizeof(PrimRecF) == 16, "primitive-pair records");
+
+__device__ __forceinline__ PrimRec ld_rec(const PrimRec* q) {
+  PrimRec r;
+  ldg32B(reinterpret_cast<const double*>(q), r.p, r.t, r.W, r.h);
+  return r;
+}
+__device__ __forceinline__ PrimRecF ld_rec(const PrimRecF* q) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(q));
+  return PrimRecF{v.x, v.y, v.z, v.w};
+}
+template <typename T>
+struct RecType;
+template <>
+struct RecType<double> {
+  using type = PrimRec;
+};
+template <>
+struct RecType<float> {
+  using type = PrimRecF;
+};
+
+// Shell pair (a, b) with la >= lb.  pp/npp index its primitive pairs
+// (contiguous); record i of the pair is at rec + i * stride().  Inside a block
+// of pairs (same class and npp) the records are primitive-major, so the lanes
+// of a warp, consecutive ket pairs, read consecutive records.
 struct __align__(16) ShellPair {
   int a, b, pp, npp;
   double Q;    // Schwarz bound sqrt(max (ab|ab))
-  int diag;    // a == b
-  int cls;     // angular pair class
+  int rec;
+  unsigned stride_diag;
+  __host__ __device__ int stride() const { return int(stride_diag >> 1); }
+  __host__ __device__ bool diag() const { return (stride_diag & 1u) != 0u; }  // a == b
 };
 
 // Work item: one bra pair against a run of at most 32 consecutive ket pairs.
@@ -69,6 +113,7 @@ struct __align__(16) Task {
 };
 
 constexpr double kTwoPi25 = 34.986836655249725693;  // 2 pi^{5/2}
+constexpr double kSqrt8Pi25 = 11.8299343455912257556;    // sqrt(8 pi^{5/2})
 
 // ---------------------------------------------------------------- E coeffs
 
@@ -177,27 +222,20 @@ struct Vec3 {
 __device__ __forceinline__ double fast_rsqrt(double x) { return rsqrt(x); }
 __device__ __forceinline__ float fast_rsqrt(float x) { return rsqrtf(x); }
 
-// Primitive-quartet scalars: fills Rn[n] = pref (-2 rho)^n F_n and R.
+// R of one primitive quartet from the exponents, W = W_ab W_cd and P - Q.
+template <typename T, int L>
+__device__ __forceinline__ void prim_quartet_R(T p, T q, T W, T PQx, T PQy, T PQz, const T* __restrict__ boys_tab,
+                                               T (&R)[nherm(L)]) {
+  T Rn[L + 1];
+  boys_hermite<T, L>(p * q, p + q, PQx * PQx + PQy * PQy + PQz * PQz, W, boys_tab, Rn);
+  hermite_R<T, L>(R, Rn, PQx, PQy, PQz);
+}
+// The same from two full primitive-pair records (1/(pq) = 4 h_p h_q).
 template <typename T, int L, typename PPT>
 __device__ __forceinline__ void prim_quartet_R(const PPT& bp, const PPT& kp, const T* __restrict__ boys_tab,
                                                T (&R)[nherm(L)]) {
-  // 1/(p+q) = r^2 with r = 1/sqrt(p+q); 1/(pq) = 4 h_p h_q: no divisions.
-  const T p = bp.p, q = kp.p;
-  const T r = fast_rsqrt(p + q);
-  const T rho = p * q * (r * r);
-  const T PQx = bp.Px - kp.Px, PQy = bp.Py - kp.Py, PQz = bp.Pz - kp.Pz;
-  const T tb = rho * (PQx * PQx + PQy * PQy + PQz * PQz);
-  T F[L + 1];
-  boys_eval<T, L>(tb, boys_tab, F);
-  T pref = T(4.0 * kTwoPi25) * T(bp.K) * T(kp.K) * (T(bp.h) * T(kp.h)) * r;
-  T Rn[L + 1];
-  const T m2rho = T(-2) * rho;
-  static_for<L + 1>([&](auto nn) {
-    constexpr int n = decltype(nn)::value;
-    Rn[n] = pref * F[n];
-    pref *= m2rho;
-  });
-  hermite_R<T, L>(R, Rn, PQx, PQy, PQz);
+  prim_quartet_R<T, L>(bp.p, kp.p, T(4.0 * kTwoPi25) * T(bp.K) * T(kp.K) * (T(bp.h) * T(kp.h)), bp.Px - kp.Px,
+                       bp.Py - kp.Py, bp.Pz - kp.Pz, boys_tab, R);
 }
 
 // Classes whose bra angular sum is at most this loop over ket primitives
@@ -205,18 +243,45 @@ __device__ __forceinline__ void prim_quartet_R(const PPT& bp, const PPT& kp, con
 // register J/K kernel can pack the kets of several bra pairs into one warp.
 constexpr int kKetOuterMaxLab = 2;
 
+// Primitive pairs of one side of a quartet: record i at rec + i * stride.
+// GLOBAL: in global memory (vector read-only loads); otherwise built on the
+// fly by the caller.
+template <typename T, bool GLOBAL>
+struct PrimList {
+  const typename RecType<T>::type* rec;
+  int stride;
+  int n;
+  __device__ __forceinline__ typename RecType<T>::type get(int i) const {
+    if constexpr (GLOBAL)
+      return ld_rec(rec + (long long)i * stride);
+    else
+      return rec[i * stride];
+  }
+};
+
+// The vectors between the centres of a quartet that its integrals depend on.
+template <typename T>
+struct QuartetGeom {
+  Vec3<T> AB, CD, CA;  // B - A, D - C, A - C
+};
+// From absolute centres; the differences are taken in FP64.
+template <typename T>
+__device__ __forceinline__ QuartetGeom<T> quartet_geom(const double* A, const double* B, const double* C,
+                                                       const double* D) {
+  return QuartetGeom<T>{Vec3<T>{T(B[0] - A[0]), T(B[1] - A[1]), T(B[2] - A[2])},
+                        Vec3<T>{T(D[0] - C[0]), T(D[1] - C[1]), T(D[2] - C[2])},
+                        Vec3<T>{T(A[0] - C[0]), T(A[1] - C[1]), T(A[2] - C[2])}};
+}
+
 // Accumulates the contracted block (ab|cd) for the ket Cartesian pairs of
 // part PART into out[ab][cdi] (cd = CD0 + cdi).  Loops over all primitive
 // pairs of the bra (outer) and ket (inner) shell pairs.  The bra E
 // coefficients live in `ebra` (3 axes); with SHARED_BRA the bra pair is the
 // same for the whole warp, `ebra` is warp-private shared memory and lanes
 // 0..2 fill one axis each (every lane of the warp must call this function).
-// GLOBAL_PP: bra/ket point into global memory (vector read-only loads);
-// false for primitive pairs built on the fly by the caller.
 template <typename T, int LA, int LB, int LC, int LD, int NS, int PART, bool SHARED_BRA, bool GLOBAL_PP = true>
 __device__ __forceinline__ void quartet_accumulate(
-    const typename PPType<T>::type* __restrict__ bra, int nbra, Vec3<T> A, Vec3<T> B,
-    const typename PPType<T>::type* __restrict__ ket, int nket, Vec3<T> C, Vec3<T> D,
+    const PrimList<T, GLOBAL_PP>& bra, const PrimList<T, GLOBAL_PP>& ket, const QuartetGeom<T>& geo,
     const T* __restrict__ boys_tab, T (*ebra)[LA + 1][LB + 1][LA + LB + 1],
     T (&out)[QCfg<LA, LB, LC, LD, NS, PART>::NAB][QCfg<LA, LB, LC, LD, NS, PART>::CDP]) {
   using Cfg = QCfg<LA, LB, LC, LD, NS, PART>;
@@ -226,12 +291,13 @@ __device__ __forceinline__ void quartet_accumulate(
     static_for<Cfg::CDP>([&](auto c) { out[decltype(ab)::value][decltype(c)::value] = T(0); });
   });
   if constexpr (Cfg::NCDP > 0) {
-    using PPT = typename PPType<T>::type;
+    using Rec = typename RecType<T>::type;
     // One primitive quartet: R, stage 1 (ket E against R) and stage 2 (bra E).
-    auto prim = [&](const PPT& bp, const EArr<T, LA, LB> Ex, const EArr<T, LA, LB> Ey, const EArr<T, LA, LB> Ez,
-                    const PPT& kp, const EArr<T, LC, LD> Fx, const EArr<T, LC, LD> Fy, const EArr<T, LC, LD> Fz) {
+    auto prim = [&](const Rec& bp, const EArr<T, LA, LB> Ex, const EArr<T, LA, LB> Ey, const EArr<T, LA, LB> Ez,
+                    const Rec& kp, const EArr<T, LC, LD> Fx, const EArr<T, LC, LD> Fy, const EArr<T, LC, LD> Fz,
+                    const Vec3<T>& PQ) {
       T R[nherm(L)];
-      prim_quartet_R<T, L>(bp, kp, boys_tab, R);
+      prim_quartet_R<T, L>(bp.p, kp.p, bp.W * kp.W, PQ.x, PQ.y, PQ.z, boys_tab, R);
       static_for<Cfg::NCDP>([&](auto cdi_) {
         constexpr int cdi = decltype(cdi_)::value;
         constexpr int cd = Cfg::CD0 + cdi, c = cd / Cfg::ND, d = cd % Cfg::ND;
@@ -282,10 +348,13 @@ __device__ __forceinline__ void quartet_accumulate(
         });
       });
     };
-    auto ket_e = [&](const PPT& kp, T (*fbuf)[LC + 1][LD + 1][LC + LD + 1]) {
-      ecoef_compute<T, LC, LD, true>(fbuf[0], kp.Px - C.x, kp.Px - D.x, kp.h);
-      ecoef_compute<T, LC, LD, true>(fbuf[1], kp.Py - C.y, kp.Py - D.y, kp.h);
-      ecoef_compute<T, LC, LD, true>(fbuf[2], kp.Pz - C.z, kp.Pz - D.z, kp.h);
+    auto ket_e = [&](const Rec& kp, T (*fbuf)[LC + 1][LD + 1][LC + LD + 1]) {
+      ecoef_compute<T, LC, LD, true>(fbuf[0], kp.t * geo.CD.x, kp.t * geo.CD.x - geo.CD.x, kp.h);
+      ecoef_compute<T, LC, LD, true>(fbuf[1], kp.t * geo.CD.y, kp.t * geo.CD.y - geo.CD.y, kp.h);
+      ecoef_compute<T, LC, LD, true>(fbuf[2], kp.t * geo.CD.z, kp.t * geo.CD.z - geo.CD.z, kp.h);
+    };
+    auto bra_e = [&](const Rec& bp, T ab, EArr<T, LA, LB> e) {
+      ecoef_compute<T, LA, LB, false>(e, bp.t * ab, bp.t * ab - ab, bp.h);
     };
     if constexpr (GLOBAL_PP && LA + LB <= kKetOuterMaxLab) {
       // Ket primitives outer: each lane reads its ket primitive pair and its
@@ -293,44 +362,45 @@ __device__ __forceinline__ void quartet_accumulate(
       // every lane: one broadcast read) and their few E coefficients are
       // redone per ket primitive in registers.  Cuts the per-lane global
       // reads of the low-L classes, which are bound by L1 throughput.
-      for (int iq = 0; iq < nket; ++iq) {
-        const PPT kp = ld_pp(ket + iq);
+      for (int iq = 0; iq < ket.n; ++iq) {
+        const Rec kp = ket.get(iq);
         T fbuf[3][LC + 1][LD + 1][LC + LD + 1];
         ket_e(kp, fbuf);
-        for (int ip = 0; ip < nbra; ++ip) {
-          const PPT bp = ld_pp(bra + ip);
+        // A - Q
+        const Vec3<T> AQ{geo.CA.x - kp.t * geo.CD.x, geo.CA.y - kp.t * geo.CD.y, geo.CA.z - kp.t * geo.CD.z};
+        for (int ip = 0; ip < bra.n; ++ip) {
+          const Rec bp = bra.get(ip);
           T eb[3][LA + 1][LB + 1][LA + LB + 1];
-          ecoef_compute<T, LA, LB, false>(eb[0], bp.Px - A.x, bp.Px - B.x, bp.h);
-          ecoef_compute<T, LA, LB, false>(eb[1], bp.Py - A.y, bp.Py - B.y, bp.h);
-          ecoef_compute<T, LA, LB, false>(eb[2], bp.Pz - A.z, bp.Pz - B.z, bp.h);
-          prim(bp, eb[0], eb[1], eb[2], kp, fbuf[0], fbuf[1], fbuf[2]);
+          bra_e(bp, geo.AB.x, eb[0]);
+          bra_e(bp, geo.AB.y, eb[1]);
+          bra_e(bp, geo.AB.z, eb[2]);
+          const Vec3<T> PQ{AQ.x + bp.t * geo.AB.x, AQ.y + bp.t * geo.AB.y, AQ.z + bp.t * geo.AB.z};
+          prim(bp, eb[0], eb[1], eb[2], kp, fbuf[0], fbuf[1], fbuf[2], PQ);
         }
       }
     } else {
       const int lane = threadIdx.x & 31;
-      for (int ip = 0; ip < nbra; ++ip) {
-        PPT bp;
-        if constexpr (GLOBAL_PP) bp = ld_pp(bra + ip);
-        else bp = bra[ip];
-        const T inv2p = bp.h;
+      for (int ip = 0; ip < bra.n; ++ip) {
+        const Rec bp = bra.get(ip);
         if constexpr (SHARED_BRA) {
           __syncwarp();
-          if (lane == 0) ecoef_compute<T, LA, LB, false>(ebra[0], bp.Px - A.x, bp.Px - B.x, inv2p);
-          if (lane == 1) ecoef_compute<T, LA, LB, false>(ebra[1], bp.Py - A.y, bp.Py - B.y, inv2p);
-          if (lane == 2) ecoef_compute<T, LA, LB, false>(ebra[2], bp.Pz - A.z, bp.Pz - B.z, inv2p);
+          if (lane == 0) bra_e(bp, geo.AB.x, ebra[0]);
+          if (lane == 1) bra_e(bp, geo.AB.y, ebra[1]);
+          if (lane == 2) bra_e(bp, geo.AB.z, ebra[2]);
           __syncwarp();
         } else {
-          ecoef_compute<T, LA, LB, false>(ebra[0], bp.Px - A.x, bp.Px - B.x, inv2p);
-          ecoef_compute<T, LA, LB, false>(ebra[1], bp.Py - A.y, bp.Py - B.y, inv2p);
-          ecoef_compute<T, LA, LB, false>(ebra[2], bp.Pz - A.z, bp.Pz - B.z, inv2p);
+          bra_e(bp, geo.AB.x, ebra[0]);
+          bra_e(bp, geo.AB.y, ebra[1]);
+          bra_e(bp, geo.AB.z, ebra[2]);
         }
-        for (int iq = 0; iq < nket; ++iq) {
-          PPT kp;
-          if constexpr (GLOBAL_PP) kp = ld_pp(ket + iq);
-          else kp = ket[iq];
+        // P - C
+        const Vec3<T> PC{geo.CA.x + bp.t * geo.AB.x, geo.CA.y + bp.t * geo.AB.y, geo.CA.z + bp.t * geo.AB.z};
+        for (int iq = 0; iq < ket.n; ++iq) {
+          const Rec kp = ket.get(iq);
           T fbuf[3][LC + 1][LD + 1][LC + LD + 1];
           ket_e(kp, fbuf);
-          prim(bp, ebra[0], ebra[1], ebra[2], kp, fbuf[0], fbuf[1], fbuf[2]);
+          const Vec3<T> PQ{PC.x - kp.t * geo.CD.x, PC.y - kp.t * geo.CD.y, PC.z - kp.t * geo.CD.z};
+          prim(bp, ebra[0], ebra[1], ebra[2], kp, fbuf[0], fbuf[1], fbuf[2], PQ);
         }
       }
     }

@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(kWarpBlock) warp_jk_kernel(const JKParams prm,
     warp_contract_pair<T>(wq, pp + bp.pp + p0, p1 - p0, centre<T>(prm.centres, bp.a), centre<T>(prm.centres, bp.b),
                           pp + kp.pp, kp.npp, centre<T>(prm.centres, kp.a), centre<T>(prm.centres, kp.b), tab);
     double s = 1.0;
-    if (bp.diag) s *= 0.5;
-    if (kp.diag) s *= 0.5;
+    if (bp.diag()) s *= 0.5;
+    if (kp.diag()) s *= 0.5;
     if (task.bra == kidx) s *= 0.5;
     warp_digest_jk<T>(prm, sm->XB, na, nb, nc, nd, prm.ao[bp.a], prm.ao[bp.b], prm.ao[kp.a], prm.ao[kp.b], s, lane);
     __syncwarp();
