@@ -285,6 +285,9 @@ struct jqc_ctx {
   TaskSet grad_tasks;  // one screened quartet per task, whole contractions
   // scratch
   DevBuf<float> d_dmax;
+  // J/K accumulator copies of the builds with 1..4 densities (jk_copies);
+  // sized by the basis, so a buffer is never replaced while graphs hold it
+  DevBuf<double> d_acc[4];
   DevBuf<double> d_pair_force;  // gradient: 6 force components per kept shell pair
   cudaStream_t side[kNumStreams] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[kNumStreams] = {};
@@ -700,18 +703,44 @@ static TaskSet* find_jk_tasks(jqc_ctx* c, int mode, double mixed_tau) {
   return nullptr;
 }
 
+// Number of copies of the J/K accumulators of a build.  The digestion's FP64
+// atomics are 14% of a full (H2O)16 build (a build without them: 5.39 of 6.24
+// ms): the warps that run at one time share a few bra rows of K, and the L2
+// slices that hold those took twice the average load.  Blocks spread over
+// copies that are summed at the end: 6.25 -> 6.06 ms with 4 ((ps|ps) 421 -> 366
+// us); 2, 8 and 16 gave 6.17, 6.06 and 6.08.  Only while the copies stay well
+// inside the L2 (126 MB); a batch's large matrices spread by themselves.
+constexpr int kJKCopies = 4;
+constexpr double kJKCopiesMaxBytes = 48e6;
+static int jk_copies(int n, int n_dens) {
+  int r = kJKCopies;
+  while (r > 1 && r * 16.0 * n_dens * n * n > kJKCopiesMaxBytes) r /= 2;
+  return r;
+}
+static size_t jk_acc_size(int n, int n_dens) { return (size_t)jk_copies(n, n_dens) * 2 * n_dens * n * n; }
+
 // One J/K build over work list `ts`: zero J/K, density maxima (when dmax is
 // given), the class kernels on the side streams (forked from and joined back
 // into s; they only add into J/K with atomics), then J = A + A^T, K = B + B^T.
 // With class_ms the classes run one after another on s, each timed.  Only
 // stream operations: no allocation, no host synchronisation except for the
 // timed form, so the untimed form can be captured into a CUDA graph.
+// own_scratch_only: no scratch of the context (the allocation-free entry).
 static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D, double* J, double* K,
-                      float* dmax, float* dmax_top, double dens_tau, cudaStream_t s, double* class_ms) {
+                      float* dmax, float* dmax_top, double dens_tau, cudaStream_t s, double* class_ms,
+                      bool own_scratch_only = false) {
   const int n = c->n_bf;
   const size_t nn = (size_t)n * n * n_dens;
-  JQC_CUDA_CHECK(cudaMemsetAsync(J, 0, nn * sizeof(double), s));
-  JQC_CUDA_CHECK(cudaMemsetAsync(K, 0, nn * sizeof(double), s));
+  const DevBuf<double>& accb = c->d_acc[n_dens - 1];
+  const int copies =
+      !own_scratch_only && accb.ptr != nullptr && accb.n >= jk_acc_size(n, n_dens) ? jk_copies(n, n_dens) : 1;
+  double* acc = copies > 1 ? accb.ptr : nullptr;  // else straight into J and K
+  if (acc != nullptr) {
+    JQC_CUDA_CHECK(cudaMemsetAsync(acc, 0, 2 * nn * copies * sizeof(double), s));
+  } else {
+    JQC_CUDA_CHECK(cudaMemsetAsync(J, 0, nn * sizeof(double), s));
+    JQC_CUDA_CHECK(cudaMemsetAsync(K, 0, nn * sizeof(double), s));
+  }
   if (class_ms)
     for (int k = 0; k < 2 * kNumQuartetClasses; ++k) class_ms[k] = 0.0;
   if (dens_tau > 0.0 && dmax != nullptr) {
@@ -749,8 +778,10 @@ static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D
       p.boys = prec ? (const void*)c->boys32 : (const void*)c->boys64;
       p.boys_al = prec ? (const void*)c->boysA32 : (const void*)c->boysA64;
       p.D = D;
-      p.J = J;
-      p.K = K;
+      p.J = acc != nullptr ? acc : J;
+      p.K = acc != nullptr ? acc + nn : K;
+      p.copies = copies;
+      p.copy_stride = (long long)(2 * nn);
       p.n = n;
       p.n_dens = n_dens;
       p.dmax = dmax;
@@ -791,8 +822,12 @@ static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D
       JQC_CUDA_CHECK(cudaStreamWaitEvent(s, c->ev_join[i], 0));
     }
   }
-  JQC_CUDA_CHECK(launch_symmetrize(J, n_dens, n, s));
-  JQC_CUDA_CHECK(launch_symmetrize(K, n_dens, n, s));
+  if (acc != nullptr) {
+    JQC_CUDA_CHECK(launch_sum_symmetrize(acc, copies, J, K, n_dens, n, s));
+  } else {
+    JQC_CUDA_CHECK(launch_symmetrize(J, n_dens, n, s));
+    JQC_CUDA_CHECK(launch_symmetrize(K, n_dens, n, s));
+  }
   return JQC_OK;
 }
 
@@ -1469,6 +1504,8 @@ static int jk_impl(jqc_ctx* c, int n_dens, const double* D, double* J, double* K
     dmax = c->d_dmax.ptr;
     dmax_top = dmax + (size_t)c->n_shell * c->n_shell;
   }
+  if (!capturing && jk_copies(c->n_bf, n_dens) > 1)
+    JQC_CUDA_CHECK(c->d_acc[n_dens - 1].reserve(jk_acc_size(c->n_bf, n_dens)));
   return run_jk_set(c, c->jk_cur, n_dens, D, J, K, dmax, dmax_top, dens_tau, s, class_ms);
 }
 
@@ -1803,7 +1840,7 @@ int jk_run_preallocated(jqc_ctx* c, int n_dens, const double* D, double* J, doub
   // the largest block maximum goes after the blocks when the scratch has room
   const size_t nb = (size_t)c->n_shell * c->n_shell;
   float* dmax_top = nb + 1 <= dmax_capacity ? dmax_scratch + nb : nullptr;
-  return run_jk_set(c, ts, n_dens, D, J, K, dmax_scratch, dmax_top, dens_tau, s, nullptr);
+  return run_jk_set(c, ts, n_dens, D, J, K, dmax_scratch, dmax_top, dens_tau, s, nullptr, true);
 }
 
 }  // namespace jqc

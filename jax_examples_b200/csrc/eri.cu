@@ -370,4 +370,45 @@ cudaError_t launch_prim_rec(const ShellPair* pairs, int n_pairs, const PrimPair*
   return cudaGetLastError();
 }
 
+// One thread per (i <= j) pair of J and of K: both triangles are written from
+// one sum.  Rows i and j of a 32 x 32 tile are read along memory through
+// shared memory.
+__global__ void __launch_bounds__(256) sum_symmetrize_kernel(const double* __restrict__ acc, int copies, int count,
+                                                             int n, double* __restrict__ J,
+                                                             double* __restrict__ K) {
+  // blockIdx.z = matrix (J matrices, then K matrices); tile (x, y) with x >= y
+  if (blockIdx.x < blockIdx.y) return;
+  __shared__ double up[32][33], lo[32][33];
+  const size_t nn = (size_t)n * n;
+  const double* M = acc + blockIdx.z * nn;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+  for (int k = ty; k < 32; k += 8) {
+    double u = 0.0, l = 0.0;
+    const bool iu = r0 + k < n && c0 + tx < n, il = c0 + k < n && r0 + tx < n;
+    for (int r = 0; r < copies; ++r) {
+      const double* Mr = M + (size_t)r * 2 * count * nn;
+      if (iu) u += Mr[(size_t)(r0 + k) * n + c0 + tx];
+      if (il) l += Mr[(size_t)(c0 + k) * n + r0 + tx];
+    }
+    up[k][tx] = u;
+    lo[k][tx] = l;
+  }
+  __syncthreads();
+  double* out = (int(blockIdx.z) < count ? J + blockIdx.z * nn : K + (blockIdx.z - count) * nn);
+  for (int k = ty; k < 32; k += 8) {
+    if (r0 + k < n && c0 + tx < n) out[(size_t)(r0 + k) * n + c0 + tx] = up[k][tx] + lo[tx][k];
+    if (blockIdx.x != blockIdx.y && c0 + k < n && r0 + tx < n)
+      out[(size_t)(c0 + k) * n + r0 + tx] = lo[k][tx] + up[tx][k];
+  }
+}
+
+cudaError_t launch_sum_symmetrize(const double* acc, int copies, double* J, double* K, int count, int n,
+                                  cudaStream_t s) {
+  if (n == 0 || count == 0) return cudaSuccess;
+  const unsigned t = unsigned((n + 31) / 32);
+  sum_symmetrize_kernel<<<dim3(t, t, unsigned(2 * count)), 256, 0, s>>>(acc, copies, count, n, J, K);
+  return cudaGetLastError();
+}
+
 }  // namespace jqc

@@ -137,8 +137,8 @@ struct JKBody {
     const int a0 = prm.ao[bp.a], b0 = prm.ao[bp.b], c0 = prm.ao[kp.a], d0 = prm.ao[kp.b];
     for (int dd = 0; dd < prm.n_dens; ++dd) {
       const double* Dm = prm.D + (size_t)dd * n * n;
-      double* Jm = prm.J + (size_t)dd * n * n;
-      double* Km = prm.K + (size_t)dd * n * n;
+      double* Jm = prm.J + jk_copy_offset(prm) + (size_t)dd * n * n;
+      double* Km = prm.K + jk_copy_offset(prm) + (size_t)dd * n * n;
       // J[a][b] (warp-uniform target): reduce over lanes first.
       double dcd[NCDP];
       static_for<NCDP>([&](auto cdi_) {

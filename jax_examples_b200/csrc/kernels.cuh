@@ -31,6 +31,10 @@ struct JKParams {
   const double* D;         // n_dens x n x n
   double* J;               // n_dens x n x n (accumulated, symmetrized later)
   double* K;
+  // Replicas of the J/K accumulators (a power of two), copy r at + r *
+  // copy_stride; block b adds into copy b mod copies.
+  int copies = 1;
+  long long copy_stride = 0;
   int n;
   int n_dens;
   const float* dmax;       // n_shell x n_shell max |D| per shell block, or null
@@ -59,6 +63,11 @@ struct JKParams {
   const int* shell_mol = nullptr;
   const int* mol_active = nullptr;
 };
+
+// Offset (in doubles) of the accumulator copy of this block.
+__device__ __forceinline__ size_t jk_copy_offset(const JKParams& p) {
+  return size_t(blockIdx.x & unsigned(p.copies - 1)) * size_t(p.copy_stride);
+}
 
 // One (precision path, class) list for the molecule compaction: its tasks,
 // its warp groups (nullptr: one task per item), the item count and where
@@ -127,6 +136,11 @@ cudaError_t launch_symmetrize(double* M, int count, int n, cudaStream_t s);
 // primitive pairs.
 cudaError_t launch_prim_rec(const ShellPair* pairs, int n_pairs, const PrimPair* pp, PrimRec* rec, PrimRecF* recf,
                             cudaStream_t s);
+// J and K (count n x n matrices each) from `copies` accumulators acc + r * 2 *
+// count * n^2, each holding the J matrices and then the K matrices: out = S +
+// S^T with S the sum of the copies.
+cudaError_t launch_sum_symmetrize(const double* acc, int copies, double* J, double* K, int count, int n,
+                                  cudaStream_t s);
 // Writes, for every segment, the indices of the work items that survive into
 // segs[k].out and their count into *segs[k].count (the counts must be zero on
 // entry).  An item survives when (with mol_active) one of its tasks belongs to

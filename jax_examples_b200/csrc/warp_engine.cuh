@@ -330,8 +330,8 @@ __device__ __forceinline__ void warp_digest_jk(const JKParams& prm, const T* blk
   const int ncd = nc * nd;
   for (int dd = 0; dd < prm.n_dens; ++dd) {
     const double* Dm = prm.D + (size_t)dd * n * n;
-    double* Jm = prm.J + (size_t)dd * n * n;
-    double* Km = prm.K + (size_t)dd * n * n;
+    double* Jm = prm.J + jk_copy_offset(prm) + (size_t)dd * n * n;
+    double* Km = prm.K + jk_copy_offset(prm) + (size_t)dd * n * n;
     for (int ab = lane; ab < na * nb; ab += 32) {
       double acc = 0.0;
       for (int cd = 0; cd < ncd; ++cd)
