@@ -20,7 +20,7 @@ constexpr int kBoysMaxM = 16;
 // Boys table: F_m(T_i), T_i = i / kBoysGridInv, m = 0 .. kBoysCols-1.
 constexpr int kBoysGridInv = 16;          // grid step 1/16
 constexpr double kBoysTMax = 36.0;        // boys_eval: table below, asymptotic above
-constexpr int kBoysTabT = 60;             // last T of the table (boys_hermite reads up to here)
+constexpr int kBoysTabT = 66;             // last T of the table (boys_hermite reads up to here)
 constexpr int kBoysRows = kBoysTabT * kBoysGridInv + 1;
 constexpr int kBoysTaylor = 8;            // Taylor terms (|dT| <= 1/32 -> ~2e-17 rel)
 constexpr int kBoysTaylorF = 5;           // FP32 Taylor terms

@@ -225,21 +225,22 @@ static int default_engine(int qc) {
 }
 static int class_engine(const ClassTune& t, int qc) { return t.engine < 0 ? default_engine(qc) : t.engine; }
 
-// Gradient: the row engine for the d-bra classes at L >= 5, the register
-// kernels up to L = 4, the warp engine otherwise.
+// Gradient engine codes: 0 (and 3, the former two-part form) the register
+// kernels of the classes with L <= 4; 1 the d-bra kernels, which are the
+// register kernels for L = 5 and 6 and the row engine for the rest; 2 the warp
+// engine.
+static bool grad_code1_class(int qc) { return qc == 11 || qc == 15 || (qc_bra(qc) >= 4 && qc_L(qc) >= 5); }
 static int default_grad_engine(int qc) {
-  if (has_grad_row_class(qc) && qc_L(qc) >= 5) return kEngineCol;
-  // dp bras in the register kernels: the split sides halve the time
-  // ((dp|ss) 4.0 -> 2.2 ms, (dp|ps) 7.4 -> 3.7 ms on (H2O)16); for the other
-  // classes computing R twice costs more than the spills it removes
-  if (is_grad_reg_class(qc) && qc_bra(qc) == 4) return kGradEngineRegSplit;
-  return is_grad_reg_class(qc) ? kEngineReg : kEngineWarp;
+  if (is_grad_reg_class(qc)) return kEngineReg;
+  return grad_code1_class(qc) ? kEngineCol : kEngineWarp;
 }
-// The register gradient kernels (one or two sides): 32 kets per task.
-static bool grad_reg_engine(int e) { return e == kEngineReg || e == kGradEngineRegSplit; }
+// Whether an engine is the register kernels (32 kets per task).
+static bool grad_reg_engine(int e, int qc) {
+  return e == kEngineReg || e == kGradEngineRegSplit || (e == kEngineCol && qc_L(qc) >= 5 && !has_grad_row_class(qc));
+}
 static bool grad_engine_valid(int e, int qc) {
   return ((e == kEngineReg || e == kGradEngineRegSplit) && is_grad_reg_class(qc)) ||
-         (e == kEngineCol && has_grad_row_class(qc)) || e == kEngineWarp;
+         (e == kEngineCol && grad_code1_class(qc)) || e == kEngineWarp;
 }
 static bool engine_valid(int e, int qc) {
   return (e == kEngineReg && is_reg_class(qc)) || (e == kEngineCol && has_col_class(qc)) || e == kEngineWarp;
@@ -298,7 +299,7 @@ struct jqc_ctx {
   const float* boysA32 = nullptr;
   double prim_tau = 0.0;
   ClassTune tune[kNumQuartetClasses];
-  int grad_engine[kNumQuartetClasses];  // JKEngine numbering: 0 register, 1 row engine, 2 warp
+  int grad_engine[kNumQuartetClasses];  // codes of jqc_set_grad_engine
   // CUDA graphs captured through jqc_graph_begin / jqc_graph_end
   std::vector<cudaGraphExec_t> graphs;
 };
@@ -383,7 +384,7 @@ static void build_task_part(const jqc_ctx* c, TaskPart& out, int g0, int g1, con
       // Register kernels: up to 32 kets per warp task (one per lane); the
       // other engines: one ket per task, so every quartet gets its own warp.
       const int per_task =
-          grad ? (grad_reg_engine(c->grad_engine[qc]) ? 32 : 1) : (class_engine(c->tune[qc], qc) == kEngineReg ? 32 : 1);
+          grad ? (grad_reg_engine(c->grad_engine[qc], qc) ? 32 : 1) : (class_engine(c->tune[qc], qc) == kEngineReg ? 32 : 1);
       for (int prec = 0; prec < 2; ++prec) {
         for (int k0 = seg[prec]; k0 < seg[prec + 1]; k0 += per_task) {
           for (int b0 = 0; b0 < nbp; b0 += chunk) {
@@ -703,6 +704,20 @@ static TaskSet* find_jk_tasks(jqc_ctx* c, int mode, double mixed_tau) {
   return nullptr;
 }
 
+// The side streams wait for s / s waits for the side streams.
+static int fork_side_streams(jqc_ctx* c, cudaStream_t s) {
+  JQC_CUDA_CHECK(cudaEventRecord(c->ev_fork, s));
+  for (int i = 0; i < kNumStreams; ++i) JQC_CUDA_CHECK(cudaStreamWaitEvent(c->side[i], c->ev_fork, 0));
+  return JQC_OK;
+}
+static int join_side_streams(jqc_ctx* c, cudaStream_t s) {
+  for (int i = 0; i < kNumStreams; ++i) {
+    JQC_CUDA_CHECK(cudaEventRecord(c->ev_join[i], c->side[i]));
+    JQC_CUDA_CHECK(cudaStreamWaitEvent(s, c->ev_join[i], 0));
+  }
+  return JQC_OK;
+}
+
 // Number of copies of the J/K accumulators of a build.  The digestion's FP64
 // atomics are 14% of a full (H2O)16 build (a build without them: 5.39 of 6.24
 // ms): the warps that run at one time share a few bra rows of K, and the L2
@@ -760,8 +775,8 @@ static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D
                                   (float)dens_tau, s));
   }
   if (!class_ms) {
-    JQC_CUDA_CHECK(cudaEventRecord(c->ev_fork, s));
-    for (int i = 0; i < kNumStreams; ++i) JQC_CUDA_CHECK(cudaStreamWaitEvent(c->side[i], c->ev_fork, 0));
+    const int rc = fork_side_streams(c, s);
+    if (rc) return rc;
   }
   int li = 0;
   for (int prec = 0; prec < 2; ++prec)
@@ -817,10 +832,8 @@ static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D
       }
     }
   if (!class_ms) {
-    for (int i = 0; i < kNumStreams; ++i) {
-      JQC_CUDA_CHECK(cudaEventRecord(c->ev_join[i], c->side[i]));
-      JQC_CUDA_CHECK(cudaStreamWaitEvent(s, c->ev_join[i], 0));
-    }
+    const int rc = join_side_streams(c, s);
+    if (rc) return rc;
   }
   if (acc != nullptr) {
     JQC_CUDA_CHECK(launch_sum_symmetrize(acc, copies, J, K, n_dens, n, s));
@@ -1378,8 +1391,7 @@ int jqc_grad2e_ex(jqc_ctx* c, int n_dens, const double* D, double j_scale, doubl
     const int pb = qc_bra(qc), pk = qc_ket(qc);
     if (class_ms) JQC_CUDA_CHECK(cudaEventRecord(c->ev_t0, s));
     const int ge = c->grad_engine[qc];
-    p.sides = ge == kGradEngineRegSplit ? 2 : 1;
-    if (grad_reg_engine(ge))
+    if (grad_reg_engine(ge, qc))
       JQC_CUDA_CHECK(launch_grad_reg(qc, p, s));
     else if (ge == kEngineCol)
       JQC_CUDA_CHECK(launch_grad_row(qc, p, s));
@@ -1600,9 +1612,8 @@ int jqc_set_grad_engine(jqc_ctx* c, int quartet_class, int engine) {
   JQC_REQUIRE(quartet_class >= 0 && quartet_class < kNumQuartetClasses, JQC_ERR_INVALID,
               "jqc_set_grad_engine: quartet class out of range");
   JQC_REQUIRE(grad_engine_valid(engine, quartet_class), JQC_ERR_INVALID,
-              "jqc_set_grad_engine: engine must be 0 (register, L <= 4), 1 (row, dp/dd bra), 2 (warp) or "
-              "3 (register, bra and ket forces in separate parts, L <= 4)");
-  const bool per_task_changed = grad_reg_engine(c->grad_engine[quartet_class]) != grad_reg_engine(engine);
+              "jqc_set_grad_engine: engine must be 0 or 3 (register, L <= 4), 1 (dp/dd bra) or 2 (warp)");
+  const bool per_task_changed = grad_reg_engine(c->grad_engine[quartet_class], quartet_class) != grad_reg_engine(engine, quartet_class);
   c->grad_engine[quartet_class] = engine;
   if (per_task_changed && c->grad_tasks.valid) {
     drop_graphs(c);

@@ -1,41 +1,87 @@
-// Register-path ERI-derivative adjoint kernel (classes with L <= 4).
+// Register-path ERI-derivative adjoint kernel (lane = ket pair).
 //
-// Same mathematics as warp_grad_kernel (grad.cu), with the class unrolled at
-// compile time and the work mapping of the J/K kernels: one warp per bra
-// pair and up to 32 ket pairs, one lane per shell quartet, blockIdx.y
-// selecting the part of the ket Cartesian pairs a thread handles.  The bra
-// E coefficients up to (la+1, lb+1) and the derivative coefficients DA, DB
-// live in warp-shared memory (the bra is warp-uniform); Gamma for the
-// thread's part, the ket E/DC coefficients, R up to L+1 and the nine force
-// components live in registers.  Forces on the bra centres are reduced over
-// the warp before the atomics; the ket centres' go straight to atomics.
+// Work mapping of the J/K kernels: one warp per bra pair and up to 32 ket
+// pairs, one lane per shell quartet, blockIdx.y selecting the part of the ket
+// Cartesian pairs a thread handles.
+//
+// Gamma is contracted with the bra's E coefficients before any integral is
+// formed.  With I = sum_abcd Gamma_abcd (ab|cd) of one primitive quartet,
+// E^{ab}_h = K e^{ab}_h(P-A, P-B, p) and the property d e^{ij}_t / d(P-A) =
+// i e^{i-1,j}_t (likewise with j for P-B), the force on the bra's centres is
+//   dI/dA = (alpha/p) dI/dP - 2 mu (A-B) I + M     mu = alpha beta / p
+//   dI/dB = (beta/p)  dI/dP + 2 mu (A-B) I - M
+//   M_x   = sum Gamma [ -(beta/p) i e^{i-1,j} + (alpha/p) j e^{i,j-1} ] ...
+// and the ket's likewise with dI/dQ = -dI/dP, so a primitive quartet needs the
+// scalar I and three vectors.  Per bra primitive pair each lane forms, for
+// its cd, the Hermite vectors
+//   H[h]   = sum_ab Gamma_abcd e^{ab}_h         HM_x[h] = the same with M_x
+// and per ket primitive pair, streaming over the bra Hermite index with
+// X[h] = sum_k e^{cd}_k R_{h+k} (never stored),
+//   I += H[h] X[h], dI/dP_x += H[h-1_x] X[h], M_x += HM_x[h] X[h],
+//   N_x += H[h] sum_k n^{cd,x}_k R_{h+k}        (the ket's M)
+// The earlier form built the derivative integrals of every ab with raised and
+// lowered E coefficients and contracted them with Gamma afterwards: five times
+// the arithmetic for a d-shell bra, 36 unrolled derivative blocks in (dd|ss).
+// (H2O)16 6-31G*, screened at 1e-9, us: (dd|ss) 1646 -> 131, (dp|ss) 951 -> 223,
+// (dp|ps) 1602 -> 442, (pp|ps) 1107 -> 276, (pp|ss) 633 -> 235, (ps|ss) 1100 ->
+// 792; with (dd|ps) 1423 -> 249, (dp|ds) 1455 -> 462 and (dp|pp) 969 -> 384,
+// which the row engine had, the classes' sum 18.1 -> 7.0 ms.  Bound by FP64
+// latency at 8 warps a multiprocessor (255 registers).
 #pragma once
 
 #include "jk_impl.cuh"
 
 namespace jqc {
 
+// Doubles a lane may hold for Gamma, H, HM of its ket Cartesian pairs and R
+// before the pairs are split over more block parts (each part evaluates R
+// again): beyond the 127 that fit in registers, but the spills of a little
+// more cost less than another R.  (H2O)16 screened / (H2O)5 gradient, ms: 80
+// 10.9 / 2.06, 100 10.6 / 2.05, 128 10.2 / 2.12, 160 10.1 / 2.18, 200 10.1 / 2.23.
+constexpr int kGradLaneDoubles = 128;
+
 __host__ __device__ constexpr int grad_split(int la, int lb, int lc, int ld) {
-  int nab = ncart(la) * ncart(lb), ncd = ncart(lc) * ncart(ld);
-  int ns = 1;
-  while (ns < 16 && nab * ((ncd + ns - 1) / ns) > 9 && ns < ncd) ns *= 2;
-  return ns;
+  const int nab = ncart(la) * ncart(lb), ncd = ncart(lc) * ncart(ld), lab = la + lb;
+  const int per = nab + nherm(lab) + (lab > 0 ? 3 * nherm(lab - 1) : 0);
+  int cdp = ncd;
+  while (cdp > 1 && cdp * per + nherm(lab + lc + ld + 1) > kGradLaneDoubles) --cdp;
+  while ((ncd + cdp - 1) / cdp > 16) ++cdp;
+  return (ncd + cdp - 1) / cdp;
 }
 
+// e^{ij}_t of the three axes and the coefficients of M.
 template <int LA, int LB>
 struct GradBraSmem {
-  double E[3][LA + 2][LB + 2][LA + LB + 3];
-  double DA[3][LA + 1][LB + 1][LA + LB + 2];
-  double DB[3][LA + 1][LB + 1][LA + LB + 2];
+  static constexpr int LAB = LA + LB;
+  double E[3][LA + 1][LB + 1][LAB + 1];
+  double M[3][LA + 1][LB + 1][LAB > 0 ? LAB : 1];  // t <= i + j - 1
 };
 
 // Decode compile-time Hermite index h into (t,u,v).
 template <int H>
 struct HermDecode {
-  static constexpr int s = (H >= 35) ? 5 : (H >= 20) ? 4 : (H >= 10) ? 3 : (H >= 4) ? 2 : (H >= 1) ? 1 : 0;
+  static constexpr int s = (H >= 84) ? 7 : (H >= 56) ? 6 : (H >= 35) ? 5 : (H >= 20) ? 4 : (H >= 10) ? 3 : (H >= 4) ? 2 : (H >= 1) ? 1 : 0;
   static constexpr int k = H - s * (s + 1) * (s + 2) / 6;
   static constexpr int t = cart_lx(s, k), u = cart_ly(s, k), v = s - t - u;
 };
+
+// m[i][j][t] = wj j e^{i,j-1}_t - wi i e^{i-1,j}_t
+template <int LI, int LJ>
+__device__ __forceinline__ void grad_m_coef(double (*m)[LJ + 1][LI + LJ > 0 ? LI + LJ : 1],
+                                            const double (*e)[LJ + 1][LI + LJ + 1], double wi, double wj) {
+  static_for<LI + 1>([&](auto i_) {
+    static_for<LJ + 1>([&](auto j_) {
+      constexpr int i = decltype(i_)::value, j = decltype(j_)::value;
+      static_for<i + j>([&](auto t_) {
+        constexpr int t = decltype(t_)::value;
+        double v = 0.0;
+        if constexpr (j > 0) v += (wj * j) * e[i][j - 1][t];
+        if constexpr (i > 0) v -= (wi * i) * e[i - 1][j][t];
+        m[i][j][t] = v;
+      });
+    });
+  });
+}
 
 template <int LA, int LB, int LC, int LD, int NS>
 struct GradBody {
@@ -43,21 +89,19 @@ struct GradBody {
   int warp, lane;
   GradBraSmem<LA, LB>* sb;
 
-  // SIDE 0: all forces; 1: bra centres (A, B) only; 2: ket centre C only.
-  template <int PART, int SIDE = 0>
+  template <int PART>
   __device__ __forceinline__ void run() {
     using Cfg = QCfg<LA, LB, LC, LD, NS, PART>;
-    if constexpr (Cfg::NCDP > 0) body<PART, SIDE>();
+    if constexpr (Cfg::NCDP > 0) body<PART>();
   }
 
-  template <int PART, int SIDE>
+  template <int PART>
   __device__ __forceinline__ void body() {
-    constexpr bool kBra = SIDE != 2, kKet = SIDE != 1;
     using Cfg = QCfg<LA, LB, LC, LD, NS, PART>;
     constexpr int NA = Cfg::NA, NB = Cfg::NB, ND = Cfg::ND;
     constexpr int NCDP = Cfg::NCDP;
     constexpr int L = Cfg::L, LAB = Cfg::LAB;
-    constexpr int NH1 = nherm(LAB + 1), NH0 = nherm(LAB);
+    constexpr int NH0 = nherm(LAB), NH1 = nherm(LAB + 1), NHM = LAB > 0 ? nherm(LAB - 1) : 0;
 
     const Task task = prm.tasks[warp];
     const ShellPair bp = prm.pairs[task.bra];
@@ -98,259 +142,218 @@ struct GradBody {
       }
       G[ab][cdi] = prm.jscale * dab * dcd - 0.5 * prm.kscale * kx;
     });
-    double g[9];
-    static_for<9>([&](auto k) { g[decltype(k)::value] = 0.0; });
+    // forces on A, on A + B (= dI/dP) and on C; D follows from translation
+    double gA[3] = {0, 0, 0}, gP[3] = {0, 0, 0}, gC[3] = {0, 0, 0};
     const int nket = active ? kp.npp : 0;
 
     const int p0 = task.flags & 0xffff, p1 = task.flags >> 16;  // bra primitive-pair range
     for (int ip = p0; ip < p1; ++ip) {
       const PrimPair bpp = ld_pp(prm.pp + bp.pp + ip);
+      const double wa = 2.0 * bpp.alpha * bpp.h, wb = 2.0 * bpp.beta * bpp.h;  // alpha / p, beta / p
       __syncwarp();
       if (lane < 3) {
         const double P = lane == 0 ? bpp.Px : lane == 1 ? bpp.Py : bpp.Pz;
         const double a = lane == 0 ? A.x : lane == 1 ? A.y : A.z;
         const double b = lane == 0 ? B.x : lane == 1 ? B.y : B.z;
-        ecoef_compute<double, LA + 1, LB + 1, false>(sb->E[lane], P - a, P - b, bpp.h);
-        static_for<LA + 1>([&](auto i_) {
-          static_for<LB + 1>([&](auto j_) {
-            static_for<LA + LB + 2>([&](auto t_) {
-              constexpr int i = decltype(i_)::value, j = decltype(j_)::value, t = decltype(t_)::value;
-              double va = 2.0 * bpp.alpha * (t <= i + 1 + j ? sb->E[lane][i + 1][j][t] : 0.0);
-              if constexpr (i > 0 && t <= i - 1 + j) va -= i * sb->E[lane][i - 1][j][t];
-              double vb = 2.0 * bpp.beta * (t <= i + j + 1 ? sb->E[lane][i][j + 1][t] : 0.0);
-              if constexpr (j > 0 && t <= i + j - 1) vb -= j * sb->E[lane][i][j - 1][t];
-              sb->DA[lane][i][j][t] = va;
-              sb->DB[lane][i][j][t] = vb;
+        ecoef_compute<double, LA, LB, false>(sb->E[lane], P - a, P - b, bpp.h);
+        grad_m_coef<LA, LB>(sb->M[lane], sb->E[lane], wb, wa);
+      }
+      __syncwarp();
+      double H[Cfg::CDP][NH0], HM[Cfg::CDP][3][NHM > 0 ? NHM : 1];
+      static_for<NCDP>([&](auto cdi_) {
+        constexpr int cdi = decltype(cdi_)::value;
+        static_for<NH0>([&](auto h_) { H[cdi][decltype(h_)::value] = 0.0; });
+        static_for<NHM>([&](auto h_) {
+          constexpr int h = decltype(h_)::value;
+          HM[cdi][0][h] = HM[cdi][1][h] = HM[cdi][2][h] = 0.0;
+        });
+      });
+      static_for<NA * NB>([&](auto ab_) {
+        constexpr int ab = decltype(ab_)::value, ia = ab / NB, ib = ab % NB;
+        constexpr int ax = cart_lx(LA, ia), ay = cart_ly(LA, ia), az = cart_lz(LA, ia);
+        constexpr int bx = cart_lx(LB, ib), by = cart_ly(LB, ib), bz = cart_lz(LB, ib);
+        static_for<ax + bx + 1>([&](auto t_) {
+          constexpr int t = decltype(t_)::value;
+          static_for<ay + by + 1>([&](auto u_) {
+            constexpr int u = decltype(u_)::value;
+            static_for<az + bz + 1>([&](auto v_) {
+              constexpr int v = decltype(v_)::value;
+              const double ex = sb->E[0][ax][bx][t], ey = sb->E[1][ay][by][u], ez = sb->E[2][az][bz][v];
+              const double e = ex * ey * ez;
+              static_for<NCDP>([&](auto c_) { H[decltype(c_)::value][herm_index(t, u, v)] += G[ab][decltype(c_)::value] * e; });
+              if constexpr (t < ax + bx) {
+                const double m = sb->M[0][ax][bx][t] * ey * ez;
+                static_for<NCDP>([&](auto c_) { HM[decltype(c_)::value][0][herm_index(t, u, v)] += G[ab][decltype(c_)::value] * m; });
+              }
+              if constexpr (u < ay + by) {
+                const double m = ex * sb->M[1][ay][by][u] * ez;
+                static_for<NCDP>([&](auto c_) { HM[decltype(c_)::value][1][herm_index(t, u, v)] += G[ab][decltype(c_)::value] * m; });
+              }
+              if constexpr (v < az + bz) {
+                const double m = ex * ey * sb->M[2][az][bz][v];
+                static_for<NCDP>([&](auto c_) { HM[decltype(c_)::value][2][herm_index(t, u, v)] += G[ab][decltype(c_)::value] * m; });
+              }
             });
           });
         });
-      }
-      __syncwarp();
+      });
+      double sI = 0.0, sP[3] = {0, 0, 0}, sM[3] = {0, 0, 0};  // over the ket primitives
       for (int iq = 0; iq < nket; ++iq) {
         const PrimPair kpp = ld_pp(prm.pp + kp.pp + iq);
-        double F[3][LC + 2][LD + 1][LC + LD + 2];
-        ecoef_compute<double, LC + 1, LD, true>(F[0], kpp.Px - C.x, kpp.Px - Dc.x, kpp.h);
-        ecoef_compute<double, LC + 1, LD, true>(F[1], kpp.Py - C.y, kpp.Py - Dc.y, kpp.h);
-        ecoef_compute<double, LC + 1, LD, true>(F[2], kpp.Pz - C.z, kpp.Pz - Dc.z, kpp.h);
+        const double wc = 2.0 * kpp.alpha * kpp.h, wd = 2.0 * kpp.beta * kpp.h;
+        double F[3][LC + 1][LD + 1][LC + LD + 1], N[3][LC + 1][LD + 1][LC + LD > 0 ? LC + LD : 1];
+        ecoef_compute<double, LC, LD, true>(F[0], kpp.Px - C.x, kpp.Px - Dc.x, kpp.h);
+        ecoef_compute<double, LC, LD, true>(F[1], kpp.Py - C.y, kpp.Py - Dc.y, kpp.h);
+        ecoef_compute<double, LC, LD, true>(F[2], kpp.Pz - C.z, kpp.Pz - Dc.z, kpp.h);
+        static_for<3>([&](auto x_) { grad_m_coef<LC, LD>(N[decltype(x_)::value], F[decltype(x_)::value], wd, wc); });
         double R[nherm(L + 1)];
         prim_quartet_R<double, L + 1>(bpp, kpp, prm.boys_al, R);
-        const double two_g = 2.0 * kpp.alpha;
-
+        double I = 0.0, dP[3] = {0, 0, 0}, n3[3] = {0, 0, 0};
         static_for<NCDP>([&](auto cdi_) {
           constexpr int cdi = decltype(cdi_)::value;
           constexpr int cd = Cfg::CD0 + cdi, c = cd / ND, d = cd % ND;
           constexpr int cx = cart_lx(LC, c), cy = cart_ly(LC, c), cz = cart_lz(LC, c);
           constexpr int dx = cart_lx(LD, d), dy = cart_ly(LD, d), dz = cart_lz(LD, d);
-          if constexpr (kBra) {
-          // stage 1 with one extra bra Hermite order
-          double X[NH1];
-          static_for<NH1>([&](auto h) { X[decltype(h)::value] = 0.0; });
-          static_for<cx + dx + 1>([&](auto tp_) {
-            constexpr int tp = decltype(tp_)::value;
-            static_for<cy + dy + 1>([&](auto up_) {
-              constexpr int up = decltype(up_)::value;
-              const double fxy = F[0][cx][dx][tp] * F[1][cy][dy][up];
-              static_for<cz + dz + 1>([&](auto vp_) {
-                constexpr int vp = decltype(vp_)::value;
-                const double f = fxy * F[2][cz][dz][vp];
-                static_for<NH1>([&](auto h_) {
-                  constexpr int h = decltype(h_)::value;
-                  using Hd = HermDecode<h>;
-                  X[h] += f * R[herm_index(Hd::t + tp, Hd::u + up, Hd::v + vp)];
-                });
-              });
+          constexpr int KX = cx + dx, KY = cy + dy, KZ = cz + dz;
+          // products of the ket coefficients for this cd
+          double fk[KX + 1][KY + 1][KZ + 1];
+          static_for<KX + 1>([&](auto t_) {
+            constexpr int t = decltype(t_)::value;
+            static_for<KY + 1>([&](auto u_) {
+              constexpr int u = decltype(u_)::value;
+              const double fxy = F[0][cx][dx][t] * F[1][cy][dy][u];
+              static_for<KZ + 1>([&](auto v_) { fk[t][u][decltype(v_)::value] = fxy * F[2][cz][dz][decltype(v_)::value]; });
             });
           });
-          // bra derivatives
-          static_for<NA * NB>([&](auto ab_) {
-            constexpr int ab = decltype(ab_)::value, ia = ab / NB, ib = ab % NB;
-            constexpr int ax = cart_lx(LA, ia), ay = cart_ly(LA, ia), az = cart_lz(LA, ia);
-            constexpr int bx = cart_lx(LB, ib), by = cart_ly(LB, ib), bz = cart_lz(LB, ib);
-            double s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0, s5 = 0;
-            // x-derivative terms: t up to ax+bx+1
-            static_for<ax + bx + 2>([&](auto t_) {
-              constexpr int t = decltype(t_)::value;
-              static_for<ay + by + 1>([&](auto u_) {
-                constexpr int u = decltype(u_)::value;
-                static_for<az + bz + 1>([&](auto v_) {
-                  constexpr int v = decltype(v_)::value;
-                  const double eyz = sb->E[1][ay][by][u] * sb->E[2][az][bz][v] * X[herm_index(t, u, v)];
-                  s0 += sb->DA[0][ax][bx][t] * eyz;
-                  s3 += sb->DB[0][ax][bx][t] * eyz;
+          static_for<NH1>([&](auto h_) {
+            constexpr int h = decltype(h_)::value;
+            using Hd = HermDecode<h>;
+            double X = 0.0;
+            static_for<KX + 1>([&](auto t_) {
+              static_for<KY + 1>([&](auto u_) {
+                static_for<KZ + 1>([&](auto v_) {
+                  constexpr int t = decltype(t_)::value, u = decltype(u_)::value, v = decltype(v_)::value;
+                  X += fk[t][u][v] * R[herm_index(Hd::t + t, Hd::u + u, Hd::v + v)];
                 });
               });
             });
-            static_for<ax + bx + 1>([&](auto t_) {
-              constexpr int t = decltype(t_)::value;
-              static_for<ay + by + 2>([&](auto u_) {
-                constexpr int u = decltype(u_)::value;
-                static_for<az + bz + 1>([&](auto v_) {
-                  constexpr int v = decltype(v_)::value;
-                  const double exz = sb->E[0][ax][bx][t] * sb->E[2][az][bz][v] * X[herm_index(t, u, v)];
-                  s1 += sb->DA[1][ay][by][u] * exz;
-                  s4 += sb->DB[1][ay][by][u] * exz;
-                });
-              });
-            });
-            static_for<ax + bx + 1>([&](auto t_) {
-              constexpr int t = decltype(t_)::value;
-              static_for<ay + by + 1>([&](auto u_) {
-                constexpr int u = decltype(u_)::value;
-                static_for<az + bz + 2>([&](auto v_) {
-                  constexpr int v = decltype(v_)::value;
-                  const double exy = sb->E[0][ax][bx][t] * sb->E[1][ay][by][u] * X[herm_index(t, u, v)];
-                  s2 += sb->DA[2][az][bz][v] * exy;
-                  s5 += sb->DB[2][az][bz][v] * exy;
-                });
-              });
-            });
-            const double w = G[ab][cdi];
-            g[0] += w * s0;
-            g[1] += w * s1;
-            g[2] += w * s2;
-            g[3] += w * s3;
-            g[4] += w * s4;
-            g[5] += w * s5;
-          });
-          }
-          // ket (centre C) derivative, one axis at a time
-          if constexpr (kKet) static_for<3>([&](auto dir_) {
-            constexpr int dir = decltype(dir_)::value;
-            constexpr int ex = cx + dx + (dir == 0), ey = cy + dy + (dir == 1), ez = cz + dz + (dir == 2);
-            double Xp[NH0];
-            static_for<NH0>([&](auto h) { Xp[decltype(h)::value] = 0.0; });
-            static_for<ex + 1>([&](auto tp_) {
-              constexpr int tp = decltype(tp_)::value;
-              static_for<ey + 1>([&](auto up_) {
-                constexpr int up = decltype(up_)::value;
-                static_for<ez + 1>([&](auto vp_) {
-                  constexpr int vp = decltype(vp_)::value;
-                  // derivative factor on axis `dir`, plain (signed) E elsewhere
-                  double fx = 0.0, fy = 0.0, fz = 0.0;
-                  if constexpr (dir == 0) {
-                    if constexpr (tp <= cx + 1 + dx) fx = two_g * F[0][cx + 1][dx][tp];
-                    if constexpr (cx > 0 && tp <= cx - 1 + dx) fx -= cx * F[0][cx - 1][dx][tp];
-                  } else if constexpr (tp <= cx + dx) {
-                    fx = F[0][cx][dx][tp];
-                  }
-                  if constexpr (dir == 1) {
-                    if constexpr (up <= cy + 1 + dy) fy = two_g * F[1][cy + 1][dy][up];
-                    if constexpr (cy > 0 && up <= cy - 1 + dy) fy -= cy * F[1][cy - 1][dy][up];
-                  } else if constexpr (up <= cy + dy) {
-                    fy = F[1][cy][dy][up];
-                  }
-                  if constexpr (dir == 2) {
-                    if constexpr (vp <= cz + 1 + dz) fz = two_g * F[2][cz + 1][dz][vp];
-                    if constexpr (cz > 0 && vp <= cz - 1 + dz) fz -= cz * F[2][cz - 1][dz][vp];
-                  } else if constexpr (vp <= cz + dz) {
-                    fz = F[2][cz][dz][vp];
-                  }
-                  const double f = fx * fy * fz;
-                  static_for<NH0>([&](auto h_) {
-                    constexpr int h = decltype(h_)::value;
-                    using Hd = HermDecode<h>;
-                    Xp[h] += f * R[herm_index(Hd::t + tp, Hd::u + up, Hd::v + vp)];
+            if constexpr (h < NH0) I += H[cdi][h] * X;
+            if constexpr (Hd::t > 0) dP[0] += H[cdi][herm_index(Hd::t > 0 ? Hd::t - 1 : 0, Hd::u, Hd::v)] * X;
+            if constexpr (Hd::u > 0) dP[1] += H[cdi][herm_index(Hd::t, Hd::u > 0 ? Hd::u - 1 : 0, Hd::v)] * X;
+            if constexpr (Hd::v > 0) dP[2] += H[cdi][herm_index(Hd::t, Hd::u, Hd::v > 0 ? Hd::v - 1 : 0)] * X;
+            if constexpr (h < NHM) {
+              sM[0] += HM[cdi][0][h] * X;
+              sM[1] += HM[cdi][1][h] * X;
+              sM[2] += HM[cdi][2][h] * X;
+            }
+            if constexpr (h < NH0) {
+              // the ket's M, one axis at a time
+              if constexpr (KX > 0) {
+                double Y = 0.0;
+                static_for<KX>([&](auto t_) {
+                  static_for<KY + 1>([&](auto u_) {
+                    static_for<KZ + 1>([&](auto v_) {
+                      constexpr int t = decltype(t_)::value, u = decltype(u_)::value, v = decltype(v_)::value;
+                      Y += N[0][cx][dx][t] * F[1][cy][dy][u] * F[2][cz][dz][v] *
+                           R[herm_index(Hd::t + t, Hd::u + u, Hd::v + v)];
+                    });
                   });
                 });
-              });
-            });
-            static_for<NA * NB>([&](auto ab_) {
-              constexpr int ab = decltype(ab_)::value, ia = ab / NB, ib = ab % NB;
-              constexpr int ax = cart_lx(LA, ia), ay = cart_ly(LA, ia), az = cart_lz(LA, ia);
-              constexpr int bx = cart_lx(LB, ib), by = cart_ly(LB, ib), bz = cart_lz(LB, ib);
-              double s = 0.0;
-              static_for<ax + bx + 1>([&](auto t_) {
-                constexpr int t = decltype(t_)::value;
-                static_for<ay + by + 1>([&](auto u_) {
-                  constexpr int u = decltype(u_)::value;
-                  const double exy = sb->E[0][ax][bx][t] * sb->E[1][ay][by][u];
-                  static_for<az + bz + 1>([&](auto v_) {
-                    constexpr int v = decltype(v_)::value;
-                    s += exy * sb->E[2][az][bz][v] * Xp[herm_index(t, u, v)];
+                n3[0] += H[cdi][h] * Y;
+              }
+              if constexpr (KY > 0) {
+                double Y = 0.0;
+                static_for<KX + 1>([&](auto t_) {
+                  static_for<KY>([&](auto u_) {
+                    static_for<KZ + 1>([&](auto v_) {
+                      constexpr int t = decltype(t_)::value, u = decltype(u_)::value, v = decltype(v_)::value;
+                      Y += F[0][cx][dx][t] * N[1][cy][dy][u] * F[2][cz][dz][v] *
+                           R[herm_index(Hd::t + t, Hd::u + u, Hd::v + v)];
+                    });
                   });
                 });
-              });
-              g[6 + dir] += G[ab][cdi] * s;
-            });
+                n3[1] += H[cdi][h] * Y;
+              }
+              if constexpr (KZ > 0) {
+                double Y = 0.0;
+                static_for<KX + 1>([&](auto t_) {
+                  static_for<KY + 1>([&](auto u_) {
+                    static_for<KZ>([&](auto v_) {
+                      constexpr int t = decltype(t_)::value, u = decltype(u_)::value, v = decltype(v_)::value;
+                      Y += F[0][cx][dx][t] * F[1][cy][dy][u] * N[2][cz][dz][v] *
+                           R[herm_index(Hd::t + t, Hd::u + u, Hd::v + v)];
+                    });
+                  });
+                });
+                n3[2] += H[cdi][h] * Y;
+              }
+            }
           });
         });
+        sI += I;
+        const double w2n = 2.0 * wc * kpp.beta;  // 2 nu
+        gC[0] += n3[0] - wc * dP[0] - w2n * (C.x - Dc.x) * I;
+        gC[1] += n3[1] - wc * dP[1] - w2n * (C.y - Dc.y) * I;
+        gC[2] += n3[2] - wc * dP[2] - w2n * (C.z - Dc.z) * I;
+        sP[0] += dP[0];
+        sP[1] += dP[1];
+        sP[2] += dP[2];
       }
+      const double w2m = 2.0 * wa * bpp.beta;  // 2 mu
+      gA[0] += sM[0] + wa * sP[0] - w2m * (A.x - B.x) * sI;
+      gA[1] += sM[1] + wa * sP[1] - w2m * (A.y - B.y) * sI;
+      gA[2] += sM[2] + wa * sP[2] - w2m * (A.z - B.z) * sI;
+      gP[0] += sP[0];
+      gP[1] += sP[1];
+      gP[2] += sP[2];
     }
     // scatter: 4 s per canonical quartet; bra centres reduced over the warp
     double sc = active ? 4.0 : 0.0;
     if (bp.diag()) sc *= 0.5;
     if (kp.diag()) sc *= 0.5;
     if (task.bra == kidx) sc *= 0.5;
-    static_for<9>([&](auto k) { g[decltype(k)::value] *= sc; });
     double* pf = prm.pair_force;
-    if constexpr (kBra) {
-      static_for<6>([&](auto k_) {
-        constexpr int k = decltype(k_)::value;
-        const double v = warp_sum(g[k]);
-        if (lane == 0) atomicAdd(pf + 6 * task.bra + k, v);
-      });
-    }
-    // centre D by translational invariance: each side adds minus its own part
+    static_for<3>([&](auto k_) {
+      constexpr int k = decltype(k_)::value;
+      const double a = warp_sum(sc * gA[k]), p = warp_sum(sc * gP[k]);
+      if (lane == 0) {
+        atomicAdd(pf + 6 * task.bra + k, a);
+        atomicAdd(pf + 6 * task.bra + 3 + k, p - a);
+      }
+    });
+    // centre D by translational invariance
     if (active) {
       static_for<3>([&](auto k_) {
         constexpr int k = decltype(k_)::value;
-        if constexpr (kKet) atomicAdd(pf + 6 * kidx + k, g[6 + k]);
-        atomicAdd(pf + 6 * kidx + 3 + k, -((kBra ? g[k] + g[3 + k] : 0.0) + (kKet ? g[6 + k] : 0.0)));
+        atomicAdd(pf + 6 * kidx + k, sc * gC[k]);
+        atomicAdd(pf + 6 * kidx + 3 + k, -sc * (gP[k] + gC[k]));
       });
     }
   }
 };
 
-// Runs one side of GradBody for the part dispatch_part selects.
-template <typename Body, int SIDE>
-struct GradSide {
-  Body& b;
-  template <int PART>
-  __device__ __forceinline__ void run() {
-    b.template run<PART, SIDE>();
-  }
-};
-
-// SIDES = 1: one block part per ket Cartesian part computes every force.
-// SIDES = 2: the bra-centre and the ket-centre forces run in separate block
-// parts (blockIdx.y = 2 * part + side), each with its own R and Boys values,
-// so a thread holds only the stage-1 sums of one side (the L = 3, 4 classes
-// otherwise spill kilobytes per thread).
-template <int LA, int LB, int LC, int LD, int SIDES>
+template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128) grad_kernel(const GradParams prm) {
   constexpr int NS = grad_split(LA, LB, LC, LD);
   __shared__ GradBraSmem<LA, LB> sB[4];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (warp >= prm.n_tasks) return;
-  using Body = GradBody<LA, LB, LC, LD, NS>;
-  Body body{prm, warp, int(threadIdx.x & 31), &sB[threadIdx.x >> 5]};
-  if constexpr (SIDES == 1) {
-    dispatch_part<NS>(blockIdx.y, body);
-  } else if (blockIdx.y & 1) {
-    GradSide<Body, 2> side{body};
-    dispatch_part<NS>(blockIdx.y >> 1, side);
-  } else {
-    GradSide<Body, 1> side{body};
-    dispatch_part<NS>(blockIdx.y >> 1, side);
-  }
+  GradBody<LA, LB, LC, LD, NS> body{prm, warp, int(threadIdx.x & 31), &sB[threadIdx.x >> 5]};
+  dispatch_part<NS>(blockIdx.y, body);
 }
 
 template <int LA, int LB, int LC, int LD>
 cudaError_t launch_grad_class(const GradParams& p, cudaStream_t s) {
   constexpr int NS = grad_split(LA, LB, LC, LD);
   if (p.n_tasks == 0) return cudaSuccess;
-  if (p.sides == 2) {
-    dim3 grid((p.n_tasks + 3) / 4, 2 * NS);
-    grad_kernel<LA, LB, LC, LD, 2><<<grid, 128, 0, s>>>(p);
-  } else {
-    dim3 grid((p.n_tasks + 3) / 4, NS);
-    grad_kernel<LA, LB, LC, LD, 1><<<grid, 128, 0, s>>>(p);
-  }
+  dim3 grid((p.n_tasks + 3) / 4, NS);
+  grad_kernel<LA, LB, LC, LD><<<grid, 128, 0, s>>>(p);
   return cudaGetLastError();
 }
 
-// Classes whose gradient runs in the register kernels, by compilation unit
-// (the unrolled classes take minutes each to compile).
+// Classes whose gradient runs in the register kernels, by compilation unit.
+// (dd|dp) and (dd|dd) were slower here (340 -> 431 and 108 -> 316 us: R to
+// order 8 and 9 does not fit a lane) and keep the row engine.
 #define JQC_FOR_GRAD_REG_SP(X) \
   X(0, 0, 0, 0, 0)             \
   X(1, 1, 0, 0, 0)             \
@@ -366,10 +369,22 @@ cudaError_t launch_grad_class(const GradParams& p, cudaStream_t s) {
 #define JQC_FOR_GRAD_REG_DP(X) \
   X(10, 2, 1, 0, 0)            \
   X(11, 2, 1, 1, 0)
-#define JQC_FOR_GRAD_REG_DD(X) X(15, 2, 2, 0, 0)
+#define JQC_FOR_GRAD_REG_DD(X) \
+  X(15, 2, 2, 0, 0)            \
+  X(16, 2, 2, 1, 0)
+#define JQC_FOR_GRAD_REG_DPPP(X) X(12, 2, 1, 1, 1)
+#define JQC_FOR_GRAD_REG_DPDS(X) X(13, 2, 1, 2, 0)
+#define JQC_FOR_GRAD_REG_DPDP(X) X(14, 2, 1, 2, 1)
+#define JQC_FOR_GRAD_REG_DDPP(X) X(17, 2, 2, 1, 1)
+#define JQC_FOR_GRAD_REG_DDDS(X) X(18, 2, 2, 2, 0)
 cudaError_t launch_grad_reg_sp(int qc, const GradParams& p, cudaStream_t s);
 cudaError_t launch_grad_reg_ds(int qc, const GradParams& p, cudaStream_t s);
 cudaError_t launch_grad_reg_dp(int qc, const GradParams& p, cudaStream_t s);
 cudaError_t launch_grad_reg_dd(int qc, const GradParams& p, cudaStream_t s);
+cudaError_t launch_grad_reg_dppp(int qc, const GradParams& p, cudaStream_t s);
+cudaError_t launch_grad_reg_dpds(int qc, const GradParams& p, cudaStream_t s);
+cudaError_t launch_grad_reg_dpdp(int qc, const GradParams& p, cudaStream_t s);
+cudaError_t launch_grad_reg_ddpp(int qc, const GradParams& p, cudaStream_t s);
+cudaError_t launch_grad_reg_ddds(int qc, const GradParams& p, cudaStream_t s);
 
 }  // namespace jqc

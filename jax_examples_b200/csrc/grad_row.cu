@@ -410,16 +410,11 @@ static cudaError_t launch_grad_row_class(const GradParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Gradient classes with a row-engine kernel (bra pair dp or dd).
+// Gradient classes with a row-engine kernel: the two it is the fastest in, and
+// the L <= 4 ones where engine code 1 asks for it.
 #define JQC_FOR_GRAD_ROW_CLASSES(X) \
   X(11, 2, 1, 1, 0)                 \
-  X(12, 2, 1, 1, 1)                 \
-  X(13, 2, 1, 2, 0)                 \
-  X(14, 2, 1, 2, 1)                 \
   X(15, 2, 2, 0, 0)                 \
-  X(16, 2, 2, 1, 0)                 \
-  X(17, 2, 2, 1, 1)                 \
-  X(18, 2, 2, 2, 0)                 \
   X(19, 2, 2, 2, 1)                 \
   X(20, 2, 2, 2, 2)
 

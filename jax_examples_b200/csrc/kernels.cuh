@@ -191,11 +191,10 @@ struct GradParams {
   const float* dmax_top = nullptr;  // the largest entry of dmax, or null
   int n_shell = 0;
   float dens_tau = 0.f;   // skip quartets whose Gamma bound x Q_ab Q_cd is below this
-  int sides = 1;          // register kernels: 2 = bra and ket forces in separate block parts
 };
 
-// Gradient engine code of the register kernels with the bra-centre and
-// ket-centre forces in separate block parts (GradParams::sides = 2).
+// Former code of the register gradient kernels with the bra-centre and ket-centre
+// forces in separate block parts: still accepted, the same kernels as code 0.
 constexpr int kGradEngineRegSplit = 3;
 
 // Upper bound of |Gamma_abcd| over a shell quartet from the per-block density
@@ -238,8 +237,7 @@ struct Grad1Params {
   double* grad;
 };
 
-// Gradient classes evaluated by the register kernels (L <= 4); the rest use
-// the warp-cooperative gradient kernel.
+// Gradient classes whose engine code 0 is the register kernels (L <= 4).
 __host__ __device__ constexpr bool is_grad_reg_class(int qc) { return qc_L(qc) <= 4; }
 cudaError_t launch_grad_reg(int qc, const GradParams& p, cudaStream_t s);
 bool has_grad_row_class(int qc);
