@@ -203,7 +203,8 @@ struct Block {
   int pc, ka, kb, start, count, mol;
 };
 
-// Upper bound on primitive quartets one lane evaluates per task (default).
+// Upper bound on primitive quartets one lane evaluates per task (default; a
+// list too short to fill the device with it takes fewer, lane_prim_limit).
 constexpr int kMaxLanePrims = 256;
 constexpr int kTuneInts = 4;  // threads, lane_prims, persistent, engine
 
@@ -253,6 +254,7 @@ using namespace jqc;
 
 struct jqc_ctx {
   int device = 0;
+  int sms = 148;
   // basis
   int n_shell = 0, n_bf = 0, n_atom = 0;
   std::vector<int> l, nprim, prim_off, ao, atom;
@@ -349,60 +351,95 @@ static int prefix_count(const std::vector<ShellPair>& pairs, int start, int limi
   return lo;
 }
 
-// Tasks and counters of the bra pairs [g0, g1) (one worker of build_tasks).
+// Surviving kets of one bra pair in one ket block: [0, n64) in FP64, [n64,
+// n_all) in FP32.
+struct KetRun {
+  int bra, block, n64, n_all;
+};
+
+// Runs, tasks and counters of the bra pairs [g0, g1) (one worker of build_tasks).
 struct TaskPart {
+  std::vector<KetRun> runs;
   std::vector<Task> lists[2][kNumQuartetClasses];
   long long nq[2] = {0, 0}, npq = 0;
   long long cq[2][kNumQuartetClasses] = {}, cp[2][kNumQuartetClasses] = {};
 };
 
-static void build_task_part(const jqc_ctx* c, TaskPart& out, int g0, int g1, const std::vector<int>& block_of,
-                            const std::vector<std::vector<int>>& mol_blocks, int mode, double mixed_tau, bool full,
-                            bool grad) {
+static void find_ket_runs(const jqc_ctx* c, TaskPart& out, int g0, int g1, const std::vector<int>& block_of,
+                          const std::vector<std::vector<int>>& mol_blocks, int mode, double mixed_tau, bool full) {
   const double tau = full ? 0.0 : c->tau;
   for (int gi = g0; gi < g1; ++gi) {
     const size_t cb = (size_t)block_of[gi];
     const Block& B = c->blocks[cb];
     const int pi = gi - B.start;
     const double Qi = c->pairs[gi].Q;
+    const int nbp = c->pairs[gi].npp;
     for (const int ckb : mol_blocks[B.mol]) {
       const size_t ck = (size_t)ckb;
       if (ck > cb) break;
       const Block& K = c->blocks[ck];
       const int limit = (ck == cb) ? pi + 1 : K.count;
       const int n_all = prefix_count(c->pairs, K.start, limit, Qi, tau);
+      if (n_all == 0) continue;
       int n64 = n_all;
       if (mode == JQC_PREC_FP32) n64 = 0;
       if (mode == JQC_PREC_MIXED) n64 = std::min(n_all, prefix_count(c->pairs, K.start, limit, Qi, mixed_tau));
       const int qc = quartet_class(B.pc, K.pc);
-      const int seg[3] = {0, n64, n_all};
-      // Split the bra primitive pairs so one lane does at most ~lane_prims
-      // primitive quartets per task (the tensor keeps whole quartets).
-      const int nbp = c->pairs[gi].npp, nkp = K.ka * K.kb;
-      int chunk = nbp;
-      if (!full) chunk = std::max(1, std::min(nbp, c->tune[qc].lane_prims / std::max(1, nkp)));
-      // Register kernels: up to 32 kets per warp task (one per lane); the
-      // other engines: one ket per task, so every quartet gets its own warp.
-      const int per_task =
-          grad ? (grad_reg_engine(c->grad_engine[qc], qc) ? 32 : 1) : (class_engine(c->tune[qc], qc) == kEngineReg ? 32 : 1);
+      const long long prims = (long long)nbp * K.ka * K.kb;
+      out.runs.push_back(KetRun{gi, ckb, n64, n_all});
+      const long long cnt[2] = {n64, n_all - n64};
       for (int prec = 0; prec < 2; ++prec) {
-        for (int k0 = seg[prec]; k0 < seg[prec + 1]; k0 += per_task) {
-          for (int b0 = 0; b0 < nbp; b0 += chunk) {
-            Task t;
-            t.bra = gi;
-            t.ket0 = K.start + k0;
-            t.nket = std::min(per_task, seg[prec + 1] - k0);
-            t.flags = b0 | (std::min(nbp, b0 + chunk) << 16);
-            out.lists[prec][qc].push_back(t);
-          }
-        }
-        out.nq[prec] += seg[prec + 1] - seg[prec];
-        out.cq[prec][qc] += seg[prec + 1] - seg[prec];
-        out.cp[prec][qc] += (long long)(seg[prec + 1] - seg[prec]) * nbp * nkp;
+        out.nq[prec] += cnt[prec];
+        out.cq[prec][qc] += cnt[prec];
+        out.cp[prec][qc] += cnt[prec] * prims;
       }
-      out.npq += (long long)n_all * c->pairs[gi].npp * K.ka * K.kb;
+      out.npq += n_all * prims;
     }
   }
+}
+
+// Primitive quartets one lane does per task: at most the class's lane_prims, and
+// fewer in a list that is short as a whole.  A lane's primitives are a serial
+// chain of 0.3 us (J/K, (ss|ss)) to 5 us (gradient, d bras) each, and the
+// classes run side by side, so the chain matters once it is a good part of the
+// whole list's time: 256 a lane made a build of one water (6-31G*) 506 us and
+// its gradient 5.1 ms, 16 a lane 256 us and 2.8 ms; (H2O)3 in 6-31G** 591 ->
+// 317 us.  Longer lists lose by short lanes (each task digests its part
+// again): (H2O)8 1.34 ms at 64 and above, 1.47 at 16; (H2O)16 7.03 at 256, 7.20
+// at 32.  The line: as many as would give each of 32 warps a multiprocessor
+// one task, over all classes.
+constexpr int kWarpsPerSM = 32;
+static int lane_prim_limit(long long prims, int lane_prims, int sms, bool grad) {
+  const int least = std::min(lane_prims, grad ? 8 : 16);
+  const long long fill = prims / (32LL * sms * kWarpsPerSM);
+  return (int)std::max<long long>(least, std::min<long long>(lane_prims, fill));
+}
+
+// The tasks of a part's runs; limit[qc] primitive quartets a lane at most
+// (the tensor keeps whole quartets), lanes[qc] kets a task at most.
+static void expand_ket_runs(const jqc_ctx* c, TaskPart& out, const std::vector<int>& block_of,
+                            const int* limit, const int* lanes, bool full) {
+  for (const KetRun& r : out.runs) {
+    const Block& K = c->blocks[r.block];
+    const Block& B = c->blocks[block_of[r.bra]];
+    const int qc = quartet_class(B.pc, K.pc);
+    const int nbp = c->pairs[r.bra].npp, nkp = K.ka * K.kb;
+    const int seg[3] = {0, r.n64, r.n_all};
+    for (int prec = 0; prec < 2; ++prec) {
+      const int chunk = full ? nbp : std::max(1, std::min(nbp, limit[qc] / std::max(1, nkp)));
+      for (int k0 = seg[prec]; k0 < seg[prec + 1]; k0 += lanes[qc]) {
+        for (int b0 = 0; b0 < nbp; b0 += chunk) {
+          Task t;
+          t.bra = r.bra;
+          t.ket0 = K.start + k0;
+          t.nket = std::min(lanes[qc], seg[prec + 1] - k0);
+          t.flags = b0 | (std::min(nbp, b0 + chunk) << 16);
+          out.lists[prec][qc].push_back(t);
+        }
+      }
+    }
+  }
+  std::vector<KetRun>().swap(out.runs);
 }
 
 // Angular momentum sum of the bra pair of quartet class qc.
@@ -467,18 +504,16 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
   int nthreads = (int)std::min<unsigned>(16u, std::max(1u, std::thread::hardware_concurrency()));
   if (n_pairs < 4096) nthreads = 1;
   std::vector<TaskPart> parts(nthreads);
-  {
+  auto each_part = [&](auto&& work) {
     std::vector<std::thread> pool;
-    for (int t = 0; t < nthreads; ++t) {
-      const int g0 = (int)((long long)n_pairs * t / nthreads), g1 = (int)((long long)n_pairs * (t + 1) / nthreads);
-      if (nthreads == 1)
-        build_task_part(c, parts[t], g0, g1, block_of, mol_blocks, mode, mixed_tau, full, grad);
-      else
-        pool.emplace_back(build_task_part, c, std::ref(parts[t]), g0, g1, std::cref(block_of), std::cref(mol_blocks),
-                          mode, mixed_tau, full, grad);
-    }
+    for (int t = 1; t < nthreads; ++t) pool.emplace_back([&work, t]() { work(t); });
+    work(0);
     for (auto& th : pool) th.join();
-  }
+  };
+  each_part([&](int t) {
+    const int g0 = (int)((long long)n_pairs * t / nthreads), g1 = (int)((long long)n_pairs * (t + 1) / nthreads);
+    find_ket_runs(c, parts[t], g0, g1, block_of, mol_blocks, mode, mixed_tau, full);
+  });
   long long nq[2] = {0, 0}, npq = 0;
   long long cq[2][kNumQuartetClasses] = {}, cp[2][kNumQuartetClasses] = {};
   for (const TaskPart& p : parts) {
@@ -491,6 +526,15 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
         cp[prec][qc] += p.cp[prec][qc];
       }
   }
+  // Register kernels: up to 32 kets per warp task (one per lane); the other
+  // engines: one ket per task, so every quartet gets its own warp.
+  int limit[kNumQuartetClasses], lanes[kNumQuartetClasses];
+  for (int qc = 0; qc < kNumQuartetClasses; ++qc) {
+    const bool reg = grad ? grad_reg_engine(c->grad_engine[qc], qc) : class_engine(c->tune[qc], qc) == kEngineReg;
+    lanes[qc] = reg ? 32 : 1;
+    limit[qc] = lane_prim_limit(npq, c->tune[qc].lane_prims, c->sms, grad);
+  }
+  each_part([&](int t) { expand_ket_runs(c, parts[t], block_of, limit, lanes, full); });
   // Every (precision path, class) list is finished on its own, the lists in
   // parallel: the parts are concatenated in bra order, the tasks ordered
   // longest first (cost = lane primitive quartets = bra primitive chunk x
@@ -879,6 +923,7 @@ int jqc_ctx_create(int device, jqc_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join[i], cudaEventDisableTiming);
   }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev_t0);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev_t1);
   if (e != cudaSuccess) {
