@@ -219,70 +219,6 @@ static cudaError_t launch_col_jk_class(const JKParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Primitive blocks (obara_saika.py:227-332 primitive_eri_block with unit
-// coefficients, K_AB and K_CD included) of the high-L classes: one warp per
-// primitive quartet, the block written back lane-strided.
-template <int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(32 * kColWarps) col_prim_kernel(const PrimQuartetParams prm) {
-  using S = ColSmem<double, LA, LB, LC, LD>;
-  extern __shared__ __align__(16) unsigned char col_smraw[];
-  S* sm = reinterpret_cast<S*>(col_smraw) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  const long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (q >= prm.n) return;
-  for (int i = lane; i < int(sizeof(sm->Fk) / sizeof(double)); i += 32) (&sm->Fk[0][0][0][0])[i] = 0.0;
-  for (int i = lane; i < int(sizeof(sm->Eb) / sizeof(double)); i += 32) (&sm->Eb[0][0][0][0])[i] = 0.0;
-  for (int i = lane; i < S::NAB * S::NCD; i += 32) sm->blk[i] = 0.0;
-  const double* ex = prm.exps + 4 * q;
-  const double* c = prm.centres + 12 * q;
-  const Vec3<double> A{c[0], c[1], c[2]}, B{c[3], c[4], c[5]}, C{c[6], c[7], c[8]}, D{c[9], c[10], c[11]};
-  PrimPair bra, ket;
-  {
-    const double al = ex[0], be = ex[1], p = al + be;
-    const double dx = A.x - B.x, dy = A.y - B.y, dz = A.z - B.z;
-    bra = PrimPair{p, 0.5 / p, (al * A.x + be * B.x) / p, (al * A.y + be * B.y) / p, (al * A.z + be * B.z) / p,
-                   exp(-(al * be / p) * (dx * dx + dy * dy + dz * dz)), al, be};
-  }
-  {
-    const double al = ex[2], be = ex[3], p = al + be;
-    const double dx = C.x - D.x, dy = C.y - D.y, dz = C.z - D.z;
-    ket = PrimPair{p, 0.5 / p, (al * C.x + be * D.x) / p, (al * C.y + be * D.y) / p, (al * C.z + be * D.z) / p,
-                   exp(-(al * be / p) * (dx * dx + dy * dy + dz * dz)), al, be};
-  }
-  __syncwarp();
-  col_set_bra<double, LA, LB, LC, LD>(sm, bra, A, B, lane);
-  col_add_prim<double, LA, LB, LC, LD>(sm, bra, ket, C, D, prm.boys, lane);
-  double* o = prm.out + q * (S::NAB * S::NCD);
-  for (int x = lane; x < S::NAB * S::NCD; x += 32) o[x] = sm->blk[x];
-}
-
-template <int LA, int LB, int LC, int LD>
-static cudaError_t launch_col_prim_class(const PrimQuartetParams& p, cudaStream_t s) {
-  if (p.n == 0) return cudaSuccess;
-  const size_t sm = kColWarps * sizeof(ColSmem<double, LA, LB, LC, LD>);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(col_prim_kernel<LA, LB, LC, LD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  const unsigned grid = (unsigned)((p.n + kColWarps - 1) / kColWarps);
-  col_prim_kernel<LA, LB, LC, LD><<<grid, 32 * kColWarps, sm, s>>>(p);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_col_prim(int qc, const PrimQuartetParams& p, cudaStream_t s) {
-  switch (qc) {
-    case 19:
-      return launch_col_prim_class<2, 2, 2, 1>(p, s);
-    case 20:
-      return launch_col_prim_class<2, 2, 2, 2>(p, s);
-    default:
-      return cudaErrorNotSupported;
-  }
-}
-
 // Classes with a column-engine kernel.
 #define JQC_FOR_COL_CLASSES(X) \
   X(12, 2, 1, 1, 1)            \

@@ -141,7 +141,7 @@ cudaError_t launch_prim_quartets(int la, int lb, int lc, int ld, const PrimQuart
   if (la < lb || lc < ld || la > 2 || lc > 2) return cudaErrorInvalidValue;
   const int pb = pair_class(la, lb), pk = pair_class(lc, ld);
   if (pb < pk) return cudaErrorInvalidValue;
-  if (!is_reg_class(quartet_class(pb, pk))) return launch_col_prim(quartet_class(pb, pk), p, s);
+  if (!is_reg_class(quartet_class(pb, pk))) return launch_prim_hi(quartet_class(pb, pk), p, s);
   switch (quartet_class(pb, pk)) {
 #define X(Q, A, B, C, D)                                                                     \
   case Q: {                                                                                  \

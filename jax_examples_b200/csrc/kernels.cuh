@@ -250,7 +250,7 @@ cudaError_t launch_pair_force_reduce(const ShellPair* pairs, int n_pairs, const 
 cudaError_t launch_warp_jk(int la, int lb, int lc, int ld, bool fp32, const JKParams& p, cudaStream_t s);
 bool has_col_class(int qc);
 cudaError_t launch_col_jk(int qc, bool fp32, const JKParams& p, cudaStream_t s);
-cudaError_t launch_col_prim(int qc, const PrimQuartetParams& p, cudaStream_t s);  // classes 19, 20
+cudaError_t launch_prim_hi(int qc, const PrimQuartetParams& p, cudaStream_t s);  // classes 19, 20
 
 cudaError_t launch_warp_tensor(int la, int lb, int lc, int ld, const TensorParams& p, cudaStream_t s);
 cudaError_t launch_warp_schwarz(int la, int lb, const SchwarzParams& p, cudaStream_t s);

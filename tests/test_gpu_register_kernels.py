@@ -1,14 +1,19 @@
-"""Edges of the register kernels' dispatch: the two sides of the Boys table's
-end, per class, against the oracle."""
+"""Edges of the quartet kernels' dispatch against the oracle: the two sides of
+the Boys table's end, ragged batches of the high-L primitive blocks, short
+work lists split over the primitives."""
 
 from __future__ import annotations
+
+import ctypes
 
 import numpy as np
 import pytest
 import torch
 
 import oracle
-from jax_examples_b200 import eri_prim_quartets
+from jax_examples_b200 import DirectERI, _abi, eri_prim_quartets
+from jax_examples_b200 import basis as pb
+from jax_examples_b200.grad import grad_two_electron
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +44,59 @@ def test_primitive_blocks_at_the_end_of_the_boys_table(cls):
         ref = oracle.primitive_eri(1.0, ctr[q, 0], cls[0], 1.0, ctr[q, 1], cls[1], 1.0, ctr[q, 2], cls[2],
                                    1.0, ctr[q, 3], cls[3], mode=1)
         np.testing.assert_allclose(got[q], ref, rtol=0, atol=tol * np.abs(ref).max(), err_msg=f"T={T[q]!r}")
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 17])
+@pytest.mark.parametrize("cls", [(2, 2, 2, 1), (2, 2, 2, 2)])
+def test_high_l_primitive_blocks_ragged(cls, n, aligned):
+    """Blocks of eight quartets: remainders, and an output array that is only
+    8-byte aligned (a C caller's).  Tolerance of the target, 1e-10 of the
+    largest element; nothing is written beyond the last block."""
+    rng = np.random.default_rng(100 * n + cls[3])
+    ex = 10 ** rng.uniform(-1, 1, (n, 4))
+    ctr = rng.uniform(0, 2.5, (n, 4, 3))
+    shape = (6, 6, 6, 6 if cls[3] == 2 else 3)
+    size = n * int(np.prod(shape))
+    buf = torch.full((size + 3,), 7.25, dtype=torch.float64, device=DEV)
+    out = buf[0 if aligned else 1:][:size]
+    e, c = (torch.tensor(x, device=DEV) for x in (ex, ctr))
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    _abi.call("jqc_eri_prim_quartets", *cls, n, ptr(e), ptr(c), ptr(out),
+              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    got = out.cpu().numpy().reshape((n,) + shape)
+    for q in range(n):
+        args = [x for k in range(4) for x in (ex[q, k], ctr[q, k], cls[k])]
+        ref = oracle.primitive_eri(*args, mode=1)
+        np.testing.assert_allclose(got[q], ref, rtol=0, atol=1e-10 * np.abs(ref).max())
+    rest = torch.cat([buf[: 0 if aligned else 1], buf[(0 if aligned else 1) + size:]])
+    assert bool((rest == 7.25).all())
+
+
+@pytest.mark.parametrize("basis,lane_prims", [("sto-3g", 1), ("6-31g*", 7), ("6-31g*", 16), ("6-31g**", 256)])
+def test_short_lists_split_over_primitives(basis, lane_prims):
+    """Lists cut into tasks of few primitives (and the limit itself, which takes
+    16 at these sizes) give the J/K and the gradient of the largest tasks to
+    1e-12: the same integrals, summed in another order."""
+    mol = pb.water_cluster(1, seed=2, noise_angstrom=0.05)
+    bs = pb.build_basis_set(mol, basis)
+    rng = np.random.default_rng(5)
+    n = bs.n_basis
+    a = rng.standard_normal((2, n, n)) * 0.1
+    D = torch.tensor(a + a.transpose(0, 2, 1), device=DEV)
+    res = []
+    for engine, lanes in ((0, lane_prims), (2, 256)):  # (2: the warp engine of the gradient)
+        eng = DirectERI(bs, mol, device=0, schwarz_tau=0.0)
+        cfg = np.zeros(84, dtype=np.int32)
+        _abi.call("jqc_get_tuning", eng._ctx, cfg.ctypes.data_as(_abi._ip))
+        cfg.reshape(21, 4)[:, 1] = lanes
+        _abi.call("jqc_set_tuning", eng._ctx, cfg.ctypes.data_as(_abi._ip))
+        if engine:
+            for q in range(21):
+                _abi.call("jqc_set_grad_engine", eng._ctx, q, engine)
+        J, K = eng.jk(D)
+        res.append((J, K, grad_two_electron(eng, list(D), 1.0, 1.0)))
+        eng.close()
+    for x, y in zip(*res):
+        scale = float(y.abs().max())
+        assert float((x - y).abs().max()) < 1e-12 * max(1.0, scale)
