@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(32 * kColWarps) col_jk_kernel(const JKParams p
   const double* ctr = prm.centres;
   const Vec3<T> A{T(ctr[3 * bp.a]), T(ctr[3 * bp.a + 1]), T(ctr[3 * bp.a + 2])};
   const Vec3<T> B{T(ctr[3 * bp.b]), T(ctr[3 * bp.b + 1]), T(ctr[3 * bp.b + 2])};
-  for (int kk = 0; kk < task.nket; ++kk) {
+  for (int kk = 0; kk < int(task.nket); ++kk) {
     const int kidx = task.ket0 + kk;
     const ShellPair kp = prm.pairs[kidx];
     if (prm.dmax_top != nullptr && float(bp.Q) * float(kp.Q) * (2.f * *prm.dmax_top) < prm.dens_tau)

@@ -246,7 +246,7 @@ static bool grad_engine_valid(int e, int qc) {
 static bool engine_valid(int e, int qc) {
   return (e == kEngineReg && is_reg_class(qc)) || (e == kEngineCol && has_col_class(qc)) || e == kEngineWarp;
 }
-constexpr int kNumStreams = 4;
+constexpr int kNumStreams = 8;  // side streams of a build (as many as the hardware's work queues)
 
 }  // namespace jqc
 
@@ -425,21 +425,34 @@ static void expand_ket_runs(const jqc_ctx* c, TaskPart& out, const std::vector<i
     const int qc = quartet_class(B.pc, K.pc);
     const int nbp = c->pairs[r.bra].npp, nkp = K.ka * K.kb;
     const int seg[3] = {0, r.n64, r.n_all};
+    const int chunk = full ? nbp : std::max(1, std::min(nbp, limit[qc] / std::max(1, nkp)));
+    // one bra primitive is still too long: the ket's are split too (a core pair
+    // has 36; (dd|ss) of one water 86 us a build with them in one lane)
+    const bool split = !full && lanes[qc] == 32 && nkp > limit[qc] && nkp < (int)Task::kAllPrims;
+    const int kchunk = split ? (nkp + (nkp + limit[qc] - 1) / limit[qc] - 1) / ((nkp + limit[qc] - 1) / limit[qc]) : nkp;
     for (int prec = 0; prec < 2; ++prec) {
-      const int chunk = full ? nbp : std::max(1, std::min(nbp, limit[qc] / std::max(1, nkp)));
       for (int k0 = seg[prec]; k0 < seg[prec + 1]; k0 += lanes[qc]) {
         for (int b0 = 0; b0 < nbp; b0 += chunk) {
-          Task t;
-          t.bra = r.bra;
-          t.ket0 = K.start + k0;
-          t.nket = std::min(lanes[qc], seg[prec + 1] - k0);
-          t.flags = b0 | (std::min(nbp, b0 + chunk) << 16);
-          out.lists[prec][qc].push_back(t);
+          for (int q0 = 0; q0 < nkp; q0 += kchunk) {
+            Task t;
+            t.bra = r.bra;
+            t.ket0 = K.start + k0;
+            t.nket = (unsigned)std::min(lanes[qc], seg[prec + 1] - k0);
+            t.q0 = (unsigned)q0;
+            t.q1 = kchunk < nkp ? (unsigned)std::min(nkp, q0 + kchunk) : Task::kAllPrims;
+            t.flags = b0 | (std::min(nbp, b0 + chunk) << 16);
+            out.lists[prec][qc].push_back(t);
+          }
         }
       }
     }
   }
   std::vector<KetRun>().swap(out.runs);
+}
+
+// Primitive quartets one lane of a task evaluates.
+static int task_lane_prims(const jqc_ctx* c, const Task& t) {
+  return ((t.flags >> 16) - (t.flags & 0xffff)) * (t.ket_end(c->pairs[t.ket0].npp) - t.ket_begin());
 }
 
 // Angular momentum sum of the bra pair of quartet class qc.
@@ -554,7 +567,7 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
       size_t k = 0;
       for (const TaskPart& p : parts)
         for (const Task& t : p.lists[prec][qc]) {
-          cost[k] = ((t.flags >> 16) - (t.flags & 0xffff)) * c->pairs[t.ket0].npp;
+          cost[k] = task_lane_prims(c, t);
           cmax = std::max(cmax, cost[k]);
           ++k;
         }
@@ -570,9 +583,8 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
         for (const Task& t : p.lists[prec][qc]) out[count[cmax - cost[k++]]++] = t;
     }
     if (!full && !grad && qc_bra_lsum(qc) <= kKetOuterMaxLab && class_engine(c->tune[qc], qc) == kEngineReg)
-      seg_ngroups[sg] = pack_groups(out, 0, total, seg_groups[sg], [c](const Task& t) {
-        return ((t.flags >> 16) - (t.flags & 0xffff)) * c->pairs[t.ket0].npp;
-      });
+      seg_ngroups[sg] =
+          pack_groups(out, 0, total, seg_groups[sg], [c](const Task& t) { return task_lane_prims(c, t); });
   };
   {
     std::vector<std::thread> pool;
@@ -748,14 +760,37 @@ static TaskSet* find_jk_tasks(jqc_ctx* c, int mode, double mixed_tau) {
   return nullptr;
 }
 
-// The side streams wait for s / s waits for the side streams.
-static int fork_side_streams(jqc_ctx* c, cudaStream_t s) {
+constexpr long long kShortListPrims = 20000000;  // see launch_order
+// Side streams for a list's kernels: two kernels each, so that a small basis
+// (six classes) does not pay for events of streams it hardly uses.  Measured
+// with 4 / 6 / 8 / 12 streams, us: (H2O)3 UHF 367 / 346 / 337 / 346, (H2O)16 mixed
+// incremental build 1704 / 1676 / 1663 / 1670, water STO-3G 59 / 61 / 64 / 64.  A
+// long gradient list keeps to four (7531 / 7553 / 7612 / 7626): its kernels
+// are all at the register limit and gain nothing from more neighbours.
+static int side_streams(const TaskSet& ts, bool grad) {
+  int lists = 0;
+  for (int k = 0; k < 2 * kNumQuartetClasses; ++k) lists += ts.cnt[k / kNumQuartetClasses][k % kNumQuartetClasses] > 0;
+  const int most = grad && ts.n_prim_quartets >= kShortListPrims ? 4 : kNumStreams;
+  return std::max(1, std::min(most, (lists + 1) / 2));
+}
+// The k-th class to launch.  In a short list the high angular momenta go first:
+// a few blocks of long, latency-bound work that the low classes fill in around
+// ((H2O)3 UHF 344 -> 319 us, (H2O)5 gradient 1.20 -> 1.15 ms).  In a long one
+// they would hold registers of multiprocessors the low classes need for
+// several waves ((H2O)16 6.15 -> 6.33 ms, its gradient 7.58 -> 7.92, 24 molecules
+// 6.69 -> 6.96).  The line, half way (as logarithms) between the (H2O)5 and
+// (H2O)16 lists, also leaves (H2O)8 (1.15 against 1.17 ms) in ascending order.
+static int launch_order(const TaskSet& ts, int k) {
+  return ts.n_prim_quartets < kShortListPrims ? kNumQuartetClasses - 1 - k : k;
+}
+// The first n side streams wait for s / s waits for them.
+static int fork_side_streams(jqc_ctx* c, cudaStream_t s, int n) {
   JQC_CUDA_CHECK(cudaEventRecord(c->ev_fork, s));
-  for (int i = 0; i < kNumStreams; ++i) JQC_CUDA_CHECK(cudaStreamWaitEvent(c->side[i], c->ev_fork, 0));
+  for (int i = 0; i < n; ++i) JQC_CUDA_CHECK(cudaStreamWaitEvent(c->side[i], c->ev_fork, 0));
   return JQC_OK;
 }
-static int join_side_streams(jqc_ctx* c, cudaStream_t s) {
-  for (int i = 0; i < kNumStreams; ++i) {
+static int join_side_streams(jqc_ctx* c, cudaStream_t s, int n) {
+  for (int i = 0; i < n; ++i) {
     JQC_CUDA_CHECK(cudaEventRecord(c->ev_join[i], c->side[i]));
     JQC_CUDA_CHECK(cudaStreamWaitEvent(s, c->ev_join[i], 0));
   }
@@ -818,13 +853,15 @@ static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D
                                   c->d_pairs.ptr, c->d_shell_mol.ptr, c->d_mol_active, dmax_top,
                                   (float)dens_tau, s));
   }
+  const int streams = side_streams(*ts, false);
   if (!class_ms) {
-    const int rc = fork_side_streams(c, s);
+    const int rc = fork_side_streams(c, s, streams);
     if (rc) return rc;
   }
   int li = 0;
   for (int prec = 0; prec < 2; ++prec)
-    for (int qc = 0; qc < kNumQuartetClasses; ++qc) {
+    for (int k = 0; k < kNumQuartetClasses; ++k) {
+      const int qc = launch_order(*ts, k);
       JKParams p;
       p.tasks = ts->d.ptr + ts->off[prec][qc];
       p.n_tasks = ts->cnt[prec][qc];
@@ -872,11 +909,11 @@ static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D
         JQC_CUDA_CHECK(cudaEventElapsedTime(&ms, c->ev_t0, c->ev_t1));
         class_ms[prec * kNumQuartetClasses + qc] = ms;
       } else {
-        JQC_CUDA_CHECK(launch_jk(qc, prec == 1, p, c->side[li++ % kNumStreams]));
+        JQC_CUDA_CHECK(launch_jk(qc, prec == 1, p, c->side[li++ % streams]));
       }
     }
   if (!class_ms) {
-    const int rc = join_side_streams(c, s);
+    const int rc = join_side_streams(c, s, streams);
     if (rc) return rc;
   }
   if (acc != nullptr) {
@@ -1414,12 +1451,14 @@ int jqc_grad2e_ex(jqc_ctx* c, int n_dens, const double* D, double j_scale, doubl
   // streams (forked from and joined back into s): one after another each
   // waits for the last block of the one before, 0.07-0.1 ms a class however
   // small ((H2O)5: 1.42 ms in a row, 21 classes).
+  const int streams = side_streams(c->grad_tasks, true);
   if (!class_ms) {
-    rc = fork_side_streams(c, s);
+    rc = fork_side_streams(c, s, streams);
     if (rc) return rc;
   }
   int li = 0;
-  for (int qc = 0; qc < kNumQuartetClasses; ++qc) {
+  for (int k = 0; k < kNumQuartetClasses; ++k) {
+    const int qc = launch_order(c->grad_tasks, k);
     GradParams p;
     p.tasks = c->grad_tasks.d.ptr + c->grad_tasks.off[0][qc];
     p.n_tasks = c->grad_tasks.cnt[0][qc];
@@ -1445,7 +1484,7 @@ int jqc_grad2e_ex(jqc_ctx* c, int n_dens, const double* D, double j_scale, doubl
     const int pb = qc_bra(qc), pk = qc_ket(qc);
     if (class_ms) JQC_CUDA_CHECK(cudaEventRecord(c->ev_t0, s));
     const int ge = c->grad_engine[qc];
-    const cudaStream_t ls = class_ms ? s : c->side[li++ % kNumStreams];
+    const cudaStream_t ls = class_ms ? s : c->side[li++ % streams];
     if (grad_reg_engine(ge, qc))
       JQC_CUDA_CHECK(launch_grad_reg(qc, p, ls));
     else if (ge == kEngineCol)
@@ -1461,7 +1500,7 @@ int jqc_grad2e_ex(jqc_ctx* c, int n_dens, const double* D, double j_scale, doubl
     }
   }
   if (!class_ms) {
-    rc = join_side_streams(c, s);
+    rc = join_side_streams(c, s, streams);
     if (rc) return rc;
   }
   JQC_CUDA_CHECK(launch_pair_force_reduce(c->d_pairs.ptr, n_pairs, c->d_atom.ptr, c->d_pair_force.ptr, grad, s));

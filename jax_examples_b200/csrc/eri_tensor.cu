@@ -23,7 +23,7 @@ struct TensorBody {
     using Cfg = QCfg<LA, LB, LC, LD, NS, PART>;
     constexpr int NA = Cfg::NA, NB = Cfg::NB, ND = Cfg::ND;
     const Task task = prm.tasks[warp];
-    const bool active = lane < task.nket;
+    const bool active = lane < int(task.nket);
     const ShellPair bp = prm.pairs[task.bra];
     const ShellPair kp = prm.pairs[task.ket0 + (active ? lane : 0)];
     const double* ctr = prm.centres;

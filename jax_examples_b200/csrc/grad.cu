@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(32 * kGradWarps, 4) warp_grad_kernel(const Gra
   const double Bx = ctr[3 * bp.b], By = ctr[3 * bp.b + 1], Bz = ctr[3 * bp.b + 2];
   const int a0 = prm.ao[bp.a], b0 = prm.ao[bp.b];
 
-  for (int kk = 0; kk < task.nket; ++kk) {
+  for (int kk = 0; kk < int(task.nket); ++kk) {
     const int kidx = task.ket0 + kk;
     const ShellPair kp = prm.pairs[kidx];
     const double Cx = ctr[3 * kp.a], Cy = ctr[3 * kp.a + 1], Cz = ctr[3 * kp.a + 2];

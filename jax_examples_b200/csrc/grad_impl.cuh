@@ -105,7 +105,7 @@ struct GradBody {
 
     const Task task = prm.tasks[warp];
     const ShellPair bp = prm.pairs[task.bra];
-    const bool in_range = lane < task.nket;
+    const bool in_range = lane < int(task.nket);
     const int kidx = task.ket0 + (in_range ? lane : 0);
     const ShellPair kp = prm.pairs[kidx];
     bool active = in_range;
@@ -144,7 +144,7 @@ struct GradBody {
     });
     // forces on A, on A + B (= dI/dP) and on C; D follows from translation
     double gA[3] = {0, 0, 0}, gP[3] = {0, 0, 0}, gC[3] = {0, 0, 0};
-    const int nket = active ? kp.npp : 0;
+    const int k0 = task.ket_begin(), k1 = active ? task.ket_end(kp.npp) : k0;  // ket primitive-pair range
 
     const int p0 = task.flags & 0xffff, p1 = task.flags >> 16;  // bra primitive-pair range
     for (int ip = p0; ip < p1; ++ip) {
@@ -198,7 +198,7 @@ struct GradBody {
         });
       });
       double sI = 0.0, sP[3] = {0, 0, 0}, sM[3] = {0, 0, 0};  // over the ket primitives
-      for (int iq = 0; iq < nket; ++iq) {
+      for (int iq = k0; iq < k1; ++iq) {
         const PrimPair kpp = ld_pp(prm.pp + kp.pp + iq);
         const double wc = 2.0 * kpp.alpha * kpp.h, wd = 2.0 * kpp.beta * kpp.h;
         double F[3][LC + 1][LD + 1][LC + LD + 1], N[3][LC + 1][LD + 1][LC + LD > 0 ? LC + LD : 1];

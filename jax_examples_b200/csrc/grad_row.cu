@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(32 * kGRowWarps, grad_row_min_blocks(LA, LB, L
   const int a0 = prm.ao[bp.a], b0 = prm.ao[bp.b];
   const int p0 = task.flags & 0xffff, p1 = task.flags >> 16;  // bra primitive-pair range
 
-  for (int kk = 0; kk < task.nket; ++kk) {
+  for (int kk = 0; kk < int(task.nket); ++kk) {
     const int kidx = task.ket0 + kk;
     const ShellPair kp = prm.pairs[kidx];
     if (prm.dmax_top != nullptr && float(bp.Q) * float(kp.Q) * gamma_bound_top(prm, *prm.dmax_top) < prm.dens_tau)

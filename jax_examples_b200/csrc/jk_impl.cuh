@@ -63,7 +63,7 @@ struct JKBody {
     if constexpr (kPacked) {
       const int g0 = prm.groups ? prm.groups[warp] : warp;
       const int nt = prm.groups ? prm.groups[warp + 1] - g0 : 1;
-      const int cnt = lane < nt ? prm.tasks[g0 + lane].nket : 0;
+      const int cnt = lane < nt ? int(prm.tasks[g0 + lane].nket) : 0;
       int incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -81,7 +81,7 @@ struct JKBody {
       seg = in_range ? ti : -1;
     } else {
       task = prm.tasks[warp];
-      in_range = lane < task.nket;
+      in_range = lane < int(task.nket);
       kidx = task.ket0 + (in_range ? lane : 0);
     }
     const ShellPair bp = prm.pairs[task.bra];
@@ -108,9 +108,10 @@ struct JKBody {
 
     T out[Cfg::NAB][Cfg::CDP];
     const int p0 = task.flags & 0xffff, p1 = task.flags >> 16;  // bra primitive-pair range
+    const int k0 = task.ket_begin(), k1 = task.ket_end(kp.npp);  // ket primitive-pair range
     quartet_accumulate<T, LA, LB, LC, LD, NS, PART, true>(
-        PrimList<T, true>{rec + bp.rec + (long long)p0 * bp.stride(), bp.stride(), p1 - p0},
-        PrimList<T, true>{rec + kp.rec, kp.stride(), active ? kp.npp : 0}, geo, static_cast<const T*>(prm.boys_al),
+        PrimList<T, true>{rec + (bp.rec + p0 * bp.stride()), bp.stride(), p1 - p0},
+        PrimList<T, true>{rec + (kp.rec + k0 * kp.stride()), kp.stride(), active ? k1 - k0 : 0}, geo, static_cast<const T*>(prm.boys_al),
         ebra, out);
 
     double s = active ? 1.0 : 0.0;

@@ -108,9 +108,18 @@ struct __align__(16) ShellPair {
 };
 
 // Work item: one bra pair against a run of at most 32 consecutive ket pairs.
+// flags: the bra's primitive pairs [flags & 0xffff, flags >> 16); q0, q1: the
+// kets' primitive pairs (register kernels only; the other engines' tasks have
+// them all).
 struct __align__(16) Task {
-  int bra, ket0, nket, flags;
+  static constexpr unsigned kAllPrims = 4095;
+  int bra, ket0;
+  unsigned nket : 8, q0 : 12, q1 : 12;
+  int flags;
+  __host__ __device__ int ket_begin() const { return int(q0); }
+  __host__ __device__ int ket_end(int npp) const { return q1 == kAllPrims ? npp : int(q1); }
 };
+static_assert(sizeof(Task) == 16, "tasks are read as one vector");
 
 constexpr double kTwoPi25 = 34.986836655249725693;  // 2 pi^{5/2}
 constexpr double kSqrt8Pi25 = 11.8299343455912257556;    // sqrt(8 pi^{5/2})
@@ -253,7 +262,7 @@ struct PrimList {
   int n;
   __device__ __forceinline__ typename RecType<T>::type get(int i) const {
     if constexpr (GLOBAL)
-      return ld_rec(rec + (long long)i * stride);
+      return ld_rec(rec + i * stride);
     else
       return rec[i * stride];
   }

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kWarpBlock) warp_jk_kernel(const JKParams prm,
   WarpQuartet<T> wq;
   wq.sm = sm;
   wq.lane = lane;
-  for (int kk = 0; kk < task.nket; ++kk) {
+  for (int kk = 0; kk < int(task.nket); ++kk) {
     const int kidx = task.ket0 + kk;
     const ShellPair kp = prm.pairs[kidx];
     if (prm.dmax_top != nullptr && float(bp.Q) * float(kp.Q) * (2.f * *prm.dmax_top) < prm.dens_tau)
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kWarpBlock) warp_tensor_kernel(const TensorPar
   WarpQuartet<double> wq;
   wq.sm = sm;
   wq.lane = lane;
-  for (int kk = 0; kk < task.nket; ++kk) {
+  for (int kk = 0; kk < int(task.nket); ++kk) {
     const ShellPair kp = prm.pairs[task.ket0 + kk];
     wq.init(la, lb, lc, ld);
     warp_contract_pair<double>(wq, prm.pp + bp.pp, bp.npp, centre<double>(prm.centres, bp.a),
