@@ -163,6 +163,42 @@ int boys_tables(int device, const double** d64, const float** d32) {
   return JQC_OK;
 }
 
+// ----------------------------------------------------------- side streams
+// Streams of destroyed contexts, kept for the next ones: creating one costs
+// about 0.11 ms, eight of them as much as the rest of a small context, and a
+// geometry optimisation makes a context for every geometry.  At most
+// kMaxIdleStreams a device stay; a stream that a capture still holds is not
+// taken back.  A reused stream may still be running work of its former owner:
+// that only orders it.
+constexpr size_t kMaxIdleStreams = 64;
+static std::mutex g_streams_mu;
+static std::vector<std::vector<cudaStream_t>> g_idle_streams;
+
+static cudaError_t take_stream(int device, cudaStream_t* out) {
+  {
+    std::lock_guard<std::mutex> lock(g_streams_mu);
+    if ((int)g_idle_streams.size() > device && !g_idle_streams[device].empty()) {
+      *out = g_idle_streams[device].back();
+      g_idle_streams[device].pop_back();
+      return cudaSuccess;
+    }
+  }
+  return cudaStreamCreateWithFlags(out, cudaStreamNonBlocking);
+}
+static void give_stream_back(int device, cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  const bool clean = cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+  if (clean) {
+    std::lock_guard<std::mutex> lock(g_streams_mu);
+    if ((int)g_idle_streams.size() <= device) g_idle_streams.resize(device + 1);
+    if (g_idle_streams[device].size() < kMaxIdleStreams) {
+      g_idle_streams[device].push_back(s);
+      return;
+    }
+  }
+  cudaStreamDestroy(s);
+}
+
 // ---------------------------------------------------------------- tasks
 struct TaskSet {
   bool valid = false;
@@ -956,7 +992,7 @@ int jqc_ctx_create(int device, jqc_ctx** out) {
   c->boysA32 = bt.a32;
   cudaError_t e = cudaSetDevice(device);
   for (int i = 0; i < kNumStreams && e == cudaSuccess; ++i) {
-    e = cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking);
+    e = take_stream(device, &c->side[i]);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join[i], cudaEventDisableTiming);
   }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
@@ -976,7 +1012,7 @@ int jqc_ctx_destroy(jqc_ctx* ctx) {
   if (ctx) {
     cudaSetDevice(ctx->device);
     for (int i = 0; i < kNumStreams; ++i) {
-      if (ctx->side[i]) cudaStreamDestroy(ctx->side[i]);
+      if (ctx->side[i]) give_stream_back(ctx->device, ctx->side[i]);
       if (ctx->ev_join[i]) cudaEventDestroy(ctx->ev_join[i]);
     }
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
@@ -1174,39 +1210,52 @@ int jqc_pairs_build(jqc_ctx* c, double schwarz_tau, double prim_tau, void* strea
     }
   c->n_pairs_all = (long long)raw.size();
   // 2. Schwarz bounds on the device
-  DevBuf<ShellPair> d_raw;
-  DevBuf<PrimPair> d_rawpp;
-  DevBuf<PrimRec> d_rawrec;
-  DevBuf<unsigned long long> d_q;
-  DevBuf<int> d_ids;
-  JQC_CUDA_CHECK(d_raw.upload(raw, s));
-  JQC_CUDA_CHECK(d_rawpp.upload(rawpp, s));
-  JQC_CUDA_CHECK(d_rawrec.reserve(rawpp.size()));
-  JQC_CUDA_CHECK(launch_prim_rec(d_raw.ptr, (int)raw.size(), d_rawpp.ptr, d_rawrec.ptr, nullptr, s));
-  JQC_CUDA_CHECK(d_q.reserve(raw.size()));
-  JQC_CUDA_CHECK(cudaMemsetAsync(d_q.ptr, 0, raw.size() * sizeof(unsigned long long), s));
+  // one temporary allocation for all of it
   std::vector<int> all_ids;
   int id_off[kNumPairClasses];
   for (int pc = 0; pc < kNumPairClasses; ++pc) {
     id_off[pc] = (int)all_ids.size();
     all_ids.insert(all_ids.end(), ids[pc].begin(), ids[pc].end());
   }
-  JQC_CUDA_CHECK(d_ids.upload(all_ids, s));
+  size_t bytes = 0;
+  auto place = [&bytes](size_t size) {
+    const size_t at = bytes;
+    bytes += (size + 255) / 256 * 256;
+    return at;
+  };
+  const size_t o_raw = place(raw.size() * sizeof(ShellPair)), o_pp = place(rawpp.size() * sizeof(PrimPair)),
+               o_rec = place(rawpp.size() * sizeof(PrimRec)), o_q = place(raw.size() * sizeof(unsigned long long)),
+               o_ids = place(all_ids.size() * sizeof(int));
+  DevBuf<unsigned char> tmp;
+  JQC_CUDA_CHECK(tmp.reserve(bytes));
+  ShellPair* const d_raw = reinterpret_cast<ShellPair*>(tmp.ptr + o_raw);
+  PrimPair* const d_rawpp = reinterpret_cast<PrimPair*>(tmp.ptr + o_pp);
+  PrimRec* const d_rawrec = reinterpret_cast<PrimRec*>(tmp.ptr + o_rec);
+  unsigned long long* const d_q = reinterpret_cast<unsigned long long*>(tmp.ptr + o_q);
+  int* const d_ids = reinterpret_cast<int*>(tmp.ptr + o_ids);
+  auto up = [s](void* dst, const void* src, size_t size) {
+    return size == 0 ? cudaSuccess : cudaMemcpyAsync(dst, src, size, cudaMemcpyHostToDevice, s);
+  };
+  JQC_CUDA_CHECK(up(d_raw, raw.data(), raw.size() * sizeof(ShellPair)));
+  JQC_CUDA_CHECK(up(d_rawpp, rawpp.data(), rawpp.size() * sizeof(PrimPair)));
+  JQC_CUDA_CHECK(up(d_ids, all_ids.data(), all_ids.size() * sizeof(int)));
+  JQC_CUDA_CHECK(launch_prim_rec(d_raw, (int)raw.size(), d_rawpp, d_rawrec, nullptr, s));
+  JQC_CUDA_CHECK(cudaMemsetAsync(d_q, 0, raw.size() * sizeof(unsigned long long), s));
   for (int pc = 0; pc < kNumPairClasses; ++pc) {
     SchwarzParams p;
-    p.pair_ids = d_ids.ptr + id_off[pc];
+    p.pair_ids = d_ids + id_off[pc];
     p.n_pairs = (int)ids[pc].size();
-    p.pairs = d_raw.ptr;
-    p.pp = d_rawpp.ptr;
-    p.rec = d_rawrec.ptr;
+    p.pairs = d_raw;
+    p.pp = d_rawpp;
+    p.rec = d_rawrec;
     p.centres = c->d_centres.ptr;
     p.boys = c->boys64;
     p.boys_al = c->boysA64;
-    p.qmax = d_q.ptr;
+    p.qmax = d_q;
     JQC_CUDA_CHECK(launch_schwarz(pc, p, s));
   }
   std::vector<unsigned long long> qbits(raw.size());
-  JQC_CUDA_CHECK(cudaMemcpyAsync(qbits.data(), d_q.ptr, qbits.size() * sizeof(unsigned long long),
+  JQC_CUDA_CHECK(cudaMemcpyAsync(qbits.data(), d_q, qbits.size() * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, s));
   JQC_CUDA_CHECK(cudaStreamSynchronize(s));
   std::vector<double> qmax(c->n_mol, 0.0);  // largest Q of each molecule

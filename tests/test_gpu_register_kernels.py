@@ -5,6 +5,7 @@ work lists split over the primitives."""
 from __future__ import annotations
 
 import ctypes
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -100,3 +101,33 @@ def test_short_lists_split_over_primitives(basis, lane_prims):
     for x, y in zip(*res):
         scale = float(y.abs().max())
         assert float((x - y).abs().max()) < 1e-12 * max(1.0, scale)
+
+
+@pytest.mark.parametrize("threads", [1, 4])
+def test_contexts_made_and_destroyed_share_side_streams(threads):
+    """Side streams outlive their context: contexts created, used and destroyed
+    one after another and in several threads at once, each thread on a stream of
+    its own, give the J/K of a fresh context (1e-12; the order of the atomics
+    differs)."""
+    mol = pb.water_cluster(2, seed=3)
+    bs = pb.build_basis_set(mol, "6-31g*")
+    n = bs.n_basis
+    a = np.random.default_rng(1).standard_normal((n, n)) * 0.1
+    D = torch.tensor(a + a.T, device=DEV)
+    eng = DirectERI(bs, mol, device=0)
+    J0, K0 = eng.jk(D)
+    torch.cuda.synchronize()
+
+    def work(_):
+        with torch.cuda.stream(torch.cuda.Stream(DEV)):
+            worst = 0.0
+            for _ in range(5):
+                e = DirectERI(bs, mol, device=0)
+                J, K = e.jk(D)
+                e.close()
+                worst = max(worst, float((J - J0).abs().max()), float((K - K0).abs().max()))
+            return worst
+
+    with ThreadPoolExecutor(threads) as ex:
+        assert max(ex.map(work, range(threads))) < 1e-12
+    eng.close()
