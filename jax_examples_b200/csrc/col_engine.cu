@@ -1,54 +1,38 @@
 // Column engine for the high angular-momentum J/K classes (L >= 5).
 //
 // One warp evaluates one contracted shell quartet (ab|cd) of a class fixed at
-// compile time; lane c owns the ket Cartesian pair cd = c (and c + 32 when a
-// class has more than 32).  Per primitive quartet:
+// compile time.  Per primitive quartet:
 //   * lanes 0..2 build the bra E coefficients of one axis each (once per bra
 //     primitive pair), lanes 3..5 the ket E (with (-1)^t), lanes 0..L the
 //     Boys values F_m(T) times the prefactor, all into the warp's slice of
 //     shared memory; the R_tuv recursion then runs in shared memory, lanes
 //     parallel over the entries of one total order;
-//   * each lane contracts its ket pair: G[h'] = F^x F^y F^z over the ket
-//     Hermite index h' (zero beyond c+d, so the loops are compile-time),
-//     X[h] = sum_h' G[h'] R[h + h'] for every bra Hermite index h (R read at
-//     the same address by all lanes: a broadcast), and
-//     block[ab][cd] += sum_tuv E^x E^y E^z X_tuv with the bra E read by all
-//     lanes at the same address.
-// Unlike the register kernels (lane = ket pair, the whole class per thread)
-// no thread holds more than the two Hermite vectors G and X, and unlike the
-// runtime-class warp engine every index is a compile-time constant.
+//   * lane h (and h + 32) owns a bra Hermite index: it reads R_{h+k} for every
+//     ket Hermite index k and turns the ket side Cartesian, X[cd][h], one axis
+//     at a time (hermite_to_cart), summed over the ket primitives.
+// Per bra primitive, lane cd reads its row X[cd][.] and turns the bra side
+// Cartesian into block[ab][cd].  The earlier form had lane = cd throughout and
+// summed over all Hermite pairs with one shared-memory read per multiply-add.
 // Digestion into J/K is the warp engine's (warp_digest_jk).
-#include "warp_engine.cuh"
+#include "axis_transform.cuh"
 
 namespace jqc {
-
-__host__ __device__ constexpr int herm_order(int h) {
-  int s = 0;
-  while (nherm(s) <= h) ++s;
-  return s;
-}
-__host__ __device__ constexpr int herm_t(int h) {
-  const int s = herm_order(h);
-  return cart_lx(s, h - nherm(s - 1));
-}
-__host__ __device__ constexpr int herm_u(int h) {
-  const int s = herm_order(h);
-  return cart_ly(s, h - nherm(s - 1));
-}
-__host__ __device__ constexpr int herm_v(int h) { return herm_order(h) - herm_t(h) - herm_u(h); }
 
 template <typename T, int LA, int LB, int LC, int LD>
 struct ColSmem {
   static constexpr int LAB = LA + LB, LCD = LC + LD, L = LAB + LCD;
   static constexpr int NAB = ncart(LA) * ncart(LB), NCD = ncart(LC) * ncart(LD);
+  static constexpr int kRow = nherm(LAB) | 1;  // odd: the rows of X on different banks
   T Eb[3][LA + 1][LB + 1][LAB + 1];
-  T Fk[3][LC + 1][LD + 1][LCD + 1];  // zero beyond t = c + d
+  T Fk[3][LC + 1][LD + 1][LCD + 1];
   T R[nherm(L)];
   T Rn[L + 1];
+  T X[NCD * kRow];
   T blk[NAB * NCD];
 };
 
 constexpr int kColWarps = 4;
+constexpr int kColSumWords = (HermSumTable::N * HermSumTable::N + 3) / 4;
 
 // Bra E coefficients of one bra primitive pair (lanes 0..2, one axis each).
 // The caller synchronises the warp before (earlier readers) and after.
@@ -60,15 +44,16 @@ __device__ __forceinline__ void col_set_bra(ColSmem<T, LA, LB, LC, LD>* sm, cons
   if (lane == 2) ecoef_compute<T, LA, LB, false>(sm->Eb[2], bp.Pz - A.z, bp.Pz - B.z, bp.h);
 }
 
-// Adds one primitive quartet (bra E already in sm->Eb) to sm->blk; all
-// lanes call with the same arguments and leave the warp synchronised.
+// One primitive quartet's X[cd][h] into sm->X (added to it unless `first`); all
+// lanes call with the same arguments and leave the warp synchronised.  `sum`:
+// kHermSum in shared memory.
 template <typename T, int LA, int LB, int LC, int LD>
 __device__ __forceinline__ void col_add_prim(ColSmem<T, LA, LB, LC, LD>* sm, const typename PPType<T>::type& bp,
                                              const typename PPType<T>::type& kp, Vec3<T> C, Vec3<T> D,
-                                             const T* __restrict__ tab, int lane) {
+                                             const T* __restrict__ tab, const unsigned char* sum, bool first,
+                                             int lane) {
   using S = ColSmem<T, LA, LB, LC, LD>;
-  constexpr int L = S::L, LAB = S::LAB, LCD = S::LCD, NCD = S::NCD;
-  constexpr int NA = ncart(LA), NB = ncart(LB), ND = ncart(LD);
+  constexpr int L = S::L, NH = nherm(S::LAB), NK = nherm(S::LCD);
   if (lane == 3) ecoef_compute<T, LC, LD, true>(sm->Fk[0], kp.Px - C.x, kp.Px - D.x, kp.h);
   if (lane == 4) ecoef_compute<T, LC, LD, true>(sm->Fk[1], kp.Py - C.y, kp.Py - D.y, kp.h);
   if (lane == 5) ecoef_compute<T, LC, LD, true>(sm->Fk[2], kp.Pz - C.z, kp.Pz - D.z, kp.h);
@@ -84,48 +69,15 @@ __device__ __forceinline__ void col_add_prim(ColSmem<T, LA, LB, LC, LD>* sm, con
   }
   __syncwarp();
   warp_hermite_R<T, L>(sm->R, sm->Rn, X, Y, Z, lane);
-  for (int c = lane; c < NCD; c += 32) {
-    const int ci = c / ND, di = c - (c / ND) * ND;
-    const int cx = cart_lx(LC, ci), cy = cart_ly(LC, ci), cz = LC - cx - cy;
-    const int dx = cart_lx(LD, di), dy = cart_ly(LD, di), dz = LD - dx - dy;
-    T G[nherm(LCD)];
-    static_for<nherm(LCD)>([&](auto h_) {
-      constexpr int h = decltype(h_)::value;
-      constexpr int ht = herm_t(h), hu = herm_u(h), hv = herm_v(h);
-      G[h] = sm->Fk[0][cx][dx][ht] * sm->Fk[1][cy][dy][hu] * sm->Fk[2][cz][dz][hv];
+  for (int h = lane; h < NH; h += 32) {
+    T rk[NK];
+    static_for<NK>([&](auto k_) {
+      constexpr int k = decltype(k_)::value;
+      rk[k] = sm->R[sum[k * HermSumTable::N + h]];
     });
-    T Xh[nherm(LAB)];
-    static_for<nherm(LAB)>([&](auto h_) {
-      constexpr int h = decltype(h_)::value;
-      constexpr int ht = herm_t(h), hu = herm_u(h), hv = herm_v(h);
-      T x = T(0);
-      static_for<nherm(LCD)>([&](auto g_) {
-        constexpr int g = decltype(g_)::value;
-        constexpr int ri = herm_index(ht + herm_t(g), hu + herm_u(g), hv + herm_v(g));
-        x += G[g] * sm->R[ri];
-      });
-      Xh[h] = x;
-    });
-    static_for<NA>([&](auto a_) {
-      constexpr int a = decltype(a_)::value;
-      constexpr int ax = cart_lx(LA, a), ay = cart_ly(LA, a), az = cart_lz(LA, a);
-      static_for<NB>([&](auto b_) {
-        constexpr int b = decltype(b_)::value;
-        constexpr int bx = cart_lx(LB, b), by = cart_ly(LB, b), bz = cart_lz(LB, b);
-        T acc = T(0);
-        static_for<ax + bx + 1>([&](auto t_) {
-          constexpr int t = decltype(t_)::value;
-          static_for<ay + by + 1>([&](auto u_) {
-            constexpr int u = decltype(u_)::value;
-            const T exy = sm->Eb[0][ax][bx][t] * sm->Eb[1][ay][by][u];
-            static_for<az + bz + 1>([&](auto v_) {
-              constexpr int v = decltype(v_)::value;
-              acc += exy * sm->Eb[2][az][bz][v] * Xh[herm_index(t, u, v)];
-            });
-          });
-        });
-        sm->blk[(a * NB + b) * NCD + c] += acc;
-      });
+    hermite_to_cart<LC, LD, 0, LC + 1>(rk, sm->Fk, [&](auto cd_, T v) {
+      T* x = sm->X + decltype(cd_)::value * S::kRow + h;
+      *x = first ? v : *x + v;
     });
   }
   __syncwarp();
@@ -136,9 +88,11 @@ __device__ __forceinline__ void col_add_prim(ColSmem<T, LA, LB, LC, LD>* sm, con
 template <typename T, int LA, int LB, int LC, int LD>
 __device__ __forceinline__ void col_quartet(ColSmem<T, LA, LB, LC, LD>* sm, const typename PPType<T>::type* bra,
                                             int nbra, Vec3<T> A, Vec3<T> B, const typename PPType<T>::type* ket,
-                                            int nket, Vec3<T> C, Vec3<T> D, const T* __restrict__ tab, int lane) {
+                                            int nket, Vec3<T> C, Vec3<T> D, const T* __restrict__ tab,
+                                            const unsigned char* sum, int lane) {
   using S = ColSmem<T, LA, LB, LC, LD>;
   using PPT = typename PPType<T>::type;
+  constexpr int NH = nherm(S::LAB), NCD = S::NCD;
   for (int i = lane; i < S::NAB * S::NCD; i += 32) sm->blk[i] = T(0);
   for (int ip = 0; ip < nbra; ++ip) {
     const PPT bp = ld_pp(bra + ip);
@@ -146,18 +100,41 @@ __device__ __forceinline__ void col_quartet(ColSmem<T, LA, LB, LC, LD>* sm, cons
     col_set_bra<T, LA, LB, LC, LD>(sm, bp, A, B, lane);
     for (int iq = 0; iq < nket; ++iq) {
       const PPT kp = ld_pp(ket + iq);
-      col_add_prim<T, LA, LB, LC, LD>(sm, bp, kp, C, D, tab, lane);
+      col_add_prim<T, LA, LB, LC, LD>(sm, bp, kp, C, D, tab, sum, iq == 0, lane);
+    }
+    if (nket == 0) continue;
+    for (int c = lane; c < NCD; c += 32) {
+      T x[NH];
+      static_for<NH>([&](auto h_) { x[decltype(h_)::value] = sm->X[c * S::kRow + decltype(h_)::value]; });
+      hermite_to_cart<LA, LB, 0, LA + 1>(x, sm->Eb,
+                                         [&](auto ab_, T v) { sm->blk[decltype(ab_)::value * NCD + c] += v; });
     }
   }
   __syncwarp();
 }
 
+// Resident blocks a multiprocessor the register allocation aims at: three (168
+// registers, 12 warps) for the FP64 (dd|dp), 270 -> 223 us in a full (H2O)16
+// build (four: 218, but 416 bytes spilled and the whole build slower); (dd|dd)
+// loses to its spills (74 -> 91 us).  Against the form with lane = cd throughout
+// and dense sums: (dd|dp) 301 -> 223 us, (dd|dd) 83 -> 74.  About 5500 warp
+// instructions a quartet, a quarter of them the digestion, at 0.3 an issue
+// slot: bound by latency and by the second lane pass for 35 Hermite functions.
+template <typename T>
+__host__ __device__ constexpr int col_min_blocks(int lc, int ld) {
+  return sizeof(T) == 8 && lc == 2 && ld == 1 ? 3 : 1;
+}
+
 template <typename T, int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(32 * kColWarps) col_jk_kernel(const JKParams prm) {
+__global__ void __launch_bounds__(32 * kColWarps, col_min_blocks<T>(LC, LD)) col_jk_kernel(const JKParams prm) {
   using S = ColSmem<T, LA, LB, LC, LD>;
   using PPT = typename PPType<T>::type;
   extern __shared__ __align__(16) unsigned char col_smraw[];
   S* sm = reinterpret_cast<S*>(col_smraw) + (threadIdx.x >> 5);
+  unsigned char* sum = col_smraw + kColWarps * sizeof(S);
+  for (int i = int(threadIdx.x); i < kColSumWords; i += int(blockDim.x))
+    reinterpret_cast<unsigned*>(sum)[i] = __ldg(reinterpret_cast<const unsigned*>(kHermSum.v) + i);
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (warp >= prm.n_tasks) return;
@@ -165,10 +142,6 @@ __global__ void __launch_bounds__(32 * kColWarps) col_jk_kernel(const JKParams p
     if (warp >= *prm.n_items) return;
     warp = prm.items[warp];
   }
-  // E entries beyond t = i + j are never written by ecoef_compute: zero them once
-  for (int i = lane; i < int(sizeof(sm->Fk) / sizeof(T)); i += 32) (&sm->Fk[0][0][0][0])[i] = T(0);
-  for (int i = lane; i < int(sizeof(sm->Eb) / sizeof(T)); i += 32) (&sm->Eb[0][0][0][0])[i] = T(0);
-  __syncwarp();
   const Task task = prm.tasks[warp];
   const ShellPair bp = prm.pairs[task.bra];
   const PPT* pp = static_cast<const PPT*>(prm.pp);
@@ -192,7 +165,7 @@ __global__ void __launch_bounds__(32 * kColWarps) col_jk_kernel(const JKParams p
     const Vec3<T> C{T(ctr[3 * kp.a]), T(ctr[3 * kp.a + 1]), T(ctr[3 * kp.a + 2])};
     const Vec3<T> Dv{T(ctr[3 * kp.b]), T(ctr[3 * kp.b + 1]), T(ctr[3 * kp.b + 2])};
     const int p0 = task.flags & 0xffff, p1 = task.flags >> 16;
-    col_quartet<T, LA, LB, LC, LD>(sm, pp + bp.pp + p0, p1 - p0, A, B, pp + kp.pp, kp.npp, C, Dv, tab, lane);
+    col_quartet<T, LA, LB, LC, LD>(sm, pp + bp.pp + p0, p1 - p0, A, B, pp + kp.pp, kp.npp, C, Dv, tab, sum, lane);
     double s = 1.0;
     if (bp.diag()) s *= 0.5;
     if (kp.diag()) s *= 0.5;
@@ -206,7 +179,7 @@ __global__ void __launch_bounds__(32 * kColWarps) col_jk_kernel(const JKParams p
 template <typename T, int LA, int LB, int LC, int LD>
 static cudaError_t launch_col_jk_class(const JKParams& p, cudaStream_t s) {
   if (p.n_tasks == 0) return cudaSuccess;
-  const size_t sm = kColWarps * sizeof(ColSmem<T, LA, LB, LC, LD>);
+  const size_t sm = kColWarps * sizeof(ColSmem<T, LA, LB, LC, LD>) + 4 * kColSumWords;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(col_jk_kernel<T, LA, LB, LC, LD>,
