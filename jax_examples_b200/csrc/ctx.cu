@@ -321,7 +321,7 @@ struct jqc_ctx {
   std::vector<TaskSet*> jk_cache;
   TaskSet* jk_cur = nullptr;
   TaskSet full_tasks;
-  TaskSet grad_tasks;  // one screened quartet per task, whole contractions
+  TaskSet grad_tasks;  // screened quartets, primitives split like the J/K lists'
   // scratch
   DevBuf<float> d_dmax;
   // J/K accumulator copies of the builds with 1..4 densities (jk_copies);
@@ -1663,8 +1663,10 @@ static int jk_impl(jqc_ctx* c, int n_dens, const double* D, double* J, double* K
     dmax = c->d_dmax.ptr;
     dmax_top = dmax + (size_t)c->n_shell * c->n_shell;
   }
-  if (!capturing && jk_copies(c->n_bf, n_dens) > 1)
-    JQC_CUDA_CHECK(c->d_acc[n_dens - 1].reserve(jk_acc_size(c->n_bf, n_dens)));
+  // Without room for the copies the build adds straight into J and K.
+  if (!capturing && jk_copies(c->n_bf, n_dens) > 1 &&
+      c->d_acc[n_dens - 1].reserve(jk_acc_size(c->n_bf, n_dens)) != cudaSuccess)
+    (void)cudaGetLastError();
   return run_jk_set(c, c->jk_cur, n_dens, D, J, K, dmax, dmax_top, dens_tau, s, class_ms);
 }
 
