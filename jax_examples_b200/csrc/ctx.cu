@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -205,7 +206,8 @@ struct TaskSet {
   int mode = -1;
   double mixed_tau = -1.0;
   bool full = false;  // no quartet screening (dense tensor)
-  std::vector<Task> h;
+  std::unique_ptr<Task[]> h;  // host copy (not initialised before the list is written)
+  size_t n_tasks = 0;
   DevBuf<Task> d;
   int off[2][kNumQuartetClasses] = {};
   int cnt[2][kNumQuartetClasses] = {};
@@ -455,17 +457,34 @@ static int lane_prim_limit(long long prims, int lane_prims, int sms, bool grad) 
 // (the tensor keeps whole quartets), lanes[qc] kets a task at most.
 static void expand_ket_runs(const jqc_ctx* c, TaskPart& out, const std::vector<int>& block_of,
                             const int* limit, const int* lanes, bool full) {
-  for (const KetRun& r : out.runs) {
+  struct Cut {
+    int qc, nbp, nkp, chunk, kchunk;
+  };
+  auto cut = [&](const KetRun& r) {
     const Block& K = c->blocks[r.block];
-    const Block& B = c->blocks[block_of[r.bra]];
-    const int qc = quartet_class(B.pc, K.pc);
+    const int qc = quartet_class(c->blocks[block_of[r.bra]].pc, K.pc);
     const int nbp = c->pairs[r.bra].npp, nkp = K.ka * K.kb;
-    const int seg[3] = {0, r.n64, r.n_all};
     const int chunk = full ? nbp : std::max(1, std::min(nbp, limit[qc] / std::max(1, nkp)));
     // one bra primitive is still too long: the ket's are split too (a core pair
     // has 36; (dd|ss) of one water 86 us a build with them in one lane)
     const bool split = !full && lanes[qc] == 32 && nkp > limit[qc] && nkp < (int)Task::kAllPrims;
     const int kchunk = split ? (nkp + (nkp + limit[qc] - 1) / limit[qc] - 1) / ((nkp + limit[qc] - 1) / limit[qc]) : nkp;
+    return Cut{qc, nbp, nkp, std::max(1, chunk), std::max(1, kchunk)};
+  };
+  size_t size[2][kNumQuartetClasses] = {};
+  for (const KetRun& r : out.runs) {
+    const Cut x = cut(r);
+    const size_t each = size_t((x.nbp + x.chunk - 1) / x.chunk) * size_t((x.nkp + x.kchunk - 1) / x.kchunk);
+    size[0][x.qc] += each * size_t((r.n64 + lanes[x.qc] - 1) / lanes[x.qc]);
+    size[1][x.qc] += each * size_t((r.n_all - r.n64 + lanes[x.qc] - 1) / lanes[x.qc]);
+  }
+  for (int prec = 0; prec < 2; ++prec)
+    for (int qc = 0; qc < kNumQuartetClasses; ++qc) out.lists[prec][qc].reserve(size[prec][qc]);
+  for (const KetRun& r : out.runs) {
+    const Block& K = c->blocks[r.block];
+    const Cut x = cut(r);
+    const int qc = x.qc, nbp = x.nbp, nkp = x.nkp, chunk = x.chunk, kchunk = x.kchunk;
+    const int seg[3] = {0, r.n64, r.n_all};
     for (int prec = 0; prec < 2; ++prec) {
       for (int k0 = seg[prec]; k0 < seg[prec + 1]; k0 += lanes[qc]) {
         for (int b0 = 0; b0 < nbp; b0 += chunk) {
@@ -494,14 +513,14 @@ static int task_lane_prims(const jqc_ctx* c, const Task& t) {
 // Angular momentum sum of the bra pair of quartet class qc.
 static int qc_bra_lsum(int qc) { return pc_la(qc_bra(qc)) + pc_lb(qc_bra(qc)); }
 
-// Packs the tasks h[base, base + n) (one class list, sorted by descending
+// Packs the tasks h[0, n) (one class list, sorted by descending
 // lane cost) into warp groups of at most 32 kets: inside each run of equal
 // cost, full tasks stay alone and the partial ones are paired largest with
 // smallest; the tasks of a group are made contiguous.  Appends the group
-// boundaries (relative to base, n_groups + 1 of them) to g and returns the
+// boundaries (n_groups + 1 of them) to g and returns the
 // number of groups.
 template <typename Cost>
-static int pack_groups(std::vector<Task>& h, size_t base, size_t n, std::vector<int>& g, Cost lane_cost) {
+static int pack_groups(Task* h, size_t n, std::vector<int>& g, Cost lane_cost) {
   std::vector<Task> part, out;
   out.reserve(n);
   int groups = 0;
@@ -509,10 +528,11 @@ static int pack_groups(std::vector<Task>& h, size_t base, size_t n, std::vector<
   size_t i0 = 0;
   while (i0 < n) {
     size_t i1 = i0;
-    while (i1 < n && lane_cost(h[base + i1]) == lane_cost(h[base + i0])) ++i1;
+    const int cost = lane_cost(h[i0]);
+    while (i1 < n && lane_cost(h[i1]) == cost) ++i1;
     part.clear();
     for (size_t k = i0; k < i1; ++k) {
-      const Task& t = h[base + k];
+      const Task& t = h[k];
       if (t.nket >= 32) {
         out.push_back(t);
         g.push_back((int)out.size());
@@ -535,7 +555,7 @@ static int pack_groups(std::vector<Task>& h, size_t base, size_t n, std::vector<
     }
     i0 = i1;
   }
-  std::copy(out.begin(), out.end(), h.begin() + (long)base);
+  std::copy(out.begin(), out.end(), h);
   return groups;
 }
 
@@ -550,8 +570,11 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
     for (int k = 0; k < c->blocks[cb].count; ++k) block_of[c->blocks[cb].start + k] = (int)cb;
   // Bra pairs split over host threads; the parts are concatenated in order,
   // so the work list does not depend on the thread count.
-  int nthreads = (int)std::min<unsigned>(16u, std::max(1u, std::thread::hardware_concurrency()));
-  if (n_pairs < 4096) nthreads = 1;
+  // A list of a few hundred pairs is done before threads have started; four
+  // take one of (H2O)3 6-31G** (first build of a geometry 1.75 -> 1.30 ms, with
+  // each list written once).
+  const int most = n_pairs < 512 ? 1 : n_pairs < 4096 ? 4 : 16;
+  const int nthreads = std::max(1, std::min(most, (int)std::thread::hardware_concurrency()));
   std::vector<TaskPart> parts(nthreads);
   auto each_part = [&](auto&& work) {
     std::vector<std::thread> pool;
@@ -590,13 +613,21 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
   // ket primitive pairs; a stable counting sort, linear in the number of
   // tasks), and the ket-outer register classes packed into warp groups.
   constexpr int kSegs = 2 * kNumQuartetClasses;
-  std::vector<std::vector<Task>> seg_tasks(kSegs);
+  size_t seg_off[kSegs + 1] = {};
+  for (int sg = 0; sg < kSegs; ++sg) {
+    seg_off[sg + 1] = seg_off[sg];
+    for (const TaskPart& p : parts) seg_off[sg + 1] += p.lists[sg / kNumQuartetClasses][sg % kNumQuartetClasses].size();
+  }
+  ts.n_tasks = seg_off[kSegs];
+  ts.h.reset(new Task[ts.n_tasks]);
+  // with each item's largest float(Q_bra) float(Q_ket), for the compaction below
+  std::vector<std::vector<float>> seg_q(kSegs);
   std::vector<std::vector<int>> seg_groups(kSegs);
   std::vector<int> seg_ngroups(kSegs, 0);
   auto finish_segment = [&](int sg) {
     const int prec = sg / kNumQuartetClasses, qc = sg % kNumQuartetClasses;
-    size_t total = 0;
-    for (const TaskPart& p : parts) total += p.lists[prec][qc].size();
+    const size_t total = seg_off[sg + 1] - seg_off[sg];
+    if (total == 0) return;
     std::vector<int> cost(total), count;
     int cmax = 0;
     {
@@ -611,8 +642,7 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
     count.assign(cmax + 2, 0);
     for (size_t k = 0; k < total; ++k) ++count[cmax - cost[k] + 1];  // descending cost
     for (int b = 1; b <= cmax + 1; ++b) count[b] += count[b - 1];
-    std::vector<Task>& out = seg_tasks[sg];
-    out.resize(total);
+    Task* const out = ts.h.get() + seg_off[sg];
     {
       size_t k = 0;
       for (const TaskPart& p : parts)
@@ -620,9 +650,26 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
     }
     if (!full && !grad && qc_bra_lsum(qc) <= kKetOuterMaxLab && class_engine(c->tune[qc], qc) == kEngineReg)
       seg_ngroups[sg] =
-          pack_groups(out, 0, total, seg_groups[sg], [c](const Task& t) { return task_lane_prims(c, t); });
+          pack_groups(out, total, seg_groups[sg], [c](const Task& t) { return task_lane_prims(c, t); });
+    if (full || grad) return;
+    auto task_q = [&](const Task& t) {
+      return float(c->pairs[t.bra].Q) * float(c->pairs[t.ket0].Q);  // ket runs: Q-descending
+    };
+    const std::vector<int>& gb = seg_groups[sg];
+    std::vector<float>& item_q = seg_q[sg];
+    item_q.resize(seg_ngroups[sg] > 0 ? (size_t)seg_ngroups[sg] : total);
+    for (size_t it = 0; it < item_q.size(); ++it) {
+      float q = 0.f;
+      if (seg_ngroups[sg] > 0)
+        for (int t = gb[it]; t < gb[it + 1]; ++t) q = std::max(q, task_q(out[t]));
+      else
+        q = task_q(out[it]);
+      item_q[it] = q;
+    }
   };
-  {
+  if (nthreads == 1) {
+    for (int sg = 0; sg < kSegs; ++sg) finish_segment(sg);
+  } else {
     std::vector<std::thread> pool;
     std::atomic<int> next{0};
     const int nw = std::max(1, std::min(nthreads, kSegs));
@@ -633,28 +680,21 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
     for (auto& th : pool) th.join();
   }
   parts.clear();
-  ts.h.clear();
   ts.gh.clear();
-  size_t total_tasks = 0, total_groups = 0;
-  for (int sg = 0; sg < kSegs; ++sg) {
-    total_tasks += seg_tasks[sg].size();
-    total_groups += seg_groups[sg].size();
-  }
-  ts.h.resize(total_tasks);
+  size_t total_groups = 0;
+  for (int sg = 0; sg < kSegs; ++sg) total_groups += seg_groups[sg].size();
   ts.gh.reserve(total_groups);
-  size_t base = 0;
   for (int sg = 0; sg < kSegs; ++sg) {
     const int prec = sg / kNumQuartetClasses, qc = sg % kNumQuartetClasses;
-    ts.off[prec][qc] = (int)base;
-    ts.cnt[prec][qc] = (int)seg_tasks[sg].size();
-    std::copy(seg_tasks[sg].begin(), seg_tasks[sg].end(), ts.h.begin() + (long)base);
-    base += seg_tasks[sg].size();
+    ts.off[prec][qc] = (int)seg_off[sg];
+    ts.cnt[prec][qc] = (int)(seg_off[sg + 1] - seg_off[sg]);
     ts.goff[prec][qc] = (int)ts.gh.size();
     ts.gcnt[prec][qc] = seg_ngroups[sg];
     ts.gh.insert(ts.gh.end(), seg_groups[sg].begin(), seg_groups[sg].end());
-    std::vector<Task>().swap(seg_tasks[sg]);
   }
-  JQC_CUDA_CHECK(ts.d.upload(ts.h, s));
+  JQC_CUDA_CHECK(ts.d.reserve(ts.n_tasks));
+  if (ts.n_tasks > 0)
+    JQC_CUDA_CHECK(cudaMemcpyAsync(ts.d.ptr, ts.h.get(), ts.n_tasks * sizeof(Task), cudaMemcpyHostToDevice, s));
   JQC_CUDA_CHECK(ts.gd.upload(ts.gh, s));
   ts.n_quartets[0] = nq[0];
   ts.n_quartets[1] = nq[1];
@@ -685,20 +725,8 @@ static int build_tasks(jqc_ctx* c, TaskSet& ts, int mode, double mixed_tau, bool
         ts.comp_item_off[nseg] = tot;
         starts.push_back(tot);
         segs.push_back(CompactSeg{nullptr, nullptr, items, nullptr, nullptr, nullptr});
-        const Task* lt = ts.h.data() + ts.off[prec][qc];
-        auto task_q = [&](const Task& t) {
-          return float(c->pairs[t.bra].Q) * float(c->pairs[t.ket0].Q);  // ket runs: Q-descending
-        };
-        for (int it = 0; it < items; ++it) {
-          float q = 0.f;
-          if (ts.gcnt[prec][qc] > 0) {
-            const int* gb = ts.gh.data() + ts.goff[prec][qc];
-            for (int t = gb[it]; t < gb[it + 1]; ++t) q = std::max(q, task_q(lt[t]));
-          } else {
-            q = task_q(lt[it]);
-          }
-          item_q.push_back(q);
-        }
+        const std::vector<float>& q = seg_q[prec * kNumQuartetClasses + qc];
+        item_q.insert(item_q.end(), q.begin(), q.end());
         tot += items;
         ++nseg;
       }
@@ -1346,7 +1374,7 @@ int jqc_stats(jqc_ctx* c, int precision_mode, double mixed_tau, long long* out) 
   int launches = 2;  // J and K symmetrization
   for (int prec = 0; prec < 2; ++prec)
     for (int qc = 0; qc < kNumQuartetClasses; ++qc) launches += c->jk_cur->cnt[prec][qc] > 0;
-  out[6] = (long long)c->jk_cur->h.size();
+  out[6] = (long long)c->jk_cur->n_tasks;
   out[7] = launches;
   return JQC_OK;
 }
