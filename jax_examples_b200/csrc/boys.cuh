@@ -185,18 +185,6 @@ __device__ __forceinline__ void boys_eval(T t, const T* __restrict__ tabA, T (&F
   }
 }
 
-// 1 / sqrt(x) for normal positive x: the hardware's approximation refined by
-// one third-order Householder step, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2
-// (the next term is 5 e^3/16).  Against rsqrt() it spares the range checks and
-// their branch.
-__device__ __forceinline__ double rsqrt_refined(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-__device__ __forceinline__ float rsqrt_refined(float x) { return rsqrtf(x); }
-
 // Where boys_hermite leaves the table: above this T the terms in e^{-T} of the
 // upward recursion are below 2^-60 of every F_m, m <= M (below 2^-30 in FP32;
 // F_0 has none, and differs from sqrt(pi/T)/2 by erfc(6) = 2e-17 at 36).
@@ -225,7 +213,7 @@ __device__ __forceinline__ void boys_hermite(T pq, T s, T R2, T W, const T* __re
   const T u = pq * R2;
   const bool near = u < T(boys_far<T>(M)) * s;
   const T x = near ? s : u;
-  const T y = rsqrt_refined(x);
+  const T y = boys_rsqrt(x);
   // 1/x by one Newton step on y^2: its powers below would multiply y's rounding
   T inv = y * y;
   inv = fma(inv, fma(-x, inv, T(1)), inv);
