@@ -96,14 +96,15 @@ struct PrimBody {
     const double* ex = prm.exps + 4 * q;
     const double* c = prm.centres + 12 * q;
     const QuartetGeom<double> geo = quartet_geom<double>(c, c + 3, c + 6, c + 9);
-    auto make = [](double al, double be, const Vec3<double>& d) {
+    // the constant of the prefactor on one side, so that it is rounded once
+    auto make = [](double al, double be, const Vec3<double>& d, double scale) {
       // one division a side; a quotient each for t and the exponent cost 51 of
       // 304 us for 2^20 (pp|pp) quartets
       const double p = al + be, inv = 1.0 / p, t = be * inv, h = 0.5 * inv;
       const double K = exp(-(al * t) * (d.x * d.x + d.y * d.y + d.z * d.z));
-      return PrimRec{p, t, K * h * kSqrt8Pi25, h};
+      return PrimRec{p, t, K * h * scale, h};
     };
-    const PrimRec bra = make(ex[0], ex[1], geo.AB), ket = make(ex[2], ex[3], geo.CD);
+    const PrimRec bra = make(ex[0], ex[1], geo.AB, 4.0 * kTwoPi25), ket = make(ex[2], ex[3], geo.CD, 1.0);
     double out[Cfg::NAB][Cfg::CDP];
     double ebuf[3][LA + 1][LB + 1][LA + LB + 1];
     quartet_accumulate<double, LA, LB, LC, LD, NS, PART, false, false>(
@@ -354,7 +355,10 @@ __global__ void __launch_bounds__(128) prim_rec_kernel(const ShellPair* __restri
   const ShellPair sp = pairs[k];
   for (int i = 0; i < sp.npp; ++i) {
     const PrimPair q = ld_pp(pp + sp.pp + i);
-    const PrimRec r{q.p, q.beta / q.p, q.K * q.h * kSqrt8Pi25, q.h};
+    // W rounded once: lo = what K h and h = 1/(2p) lost.  A pair's W is in all of its
+    // integrals, so its rounding does not average out.
+    const double Kh = q.K * q.h, lo = fma(q.K, q.h, -Kh) + Kh * fma(-2.0 * q.p, q.h, 1.0);
+    const PrimRec r{q.p, q.beta / q.p, fma(Kh, kSqrt8Pi25, fma(Kh, kSqrt8Pi25Lo, lo * kSqrt8Pi25)), q.h};
     const long long at = sp.rec + (long long)i * sp.stride();
     rec[at] = r;
     if (recf != nullptr) recf[at] = PrimRecF{float(r.p), float(r.t), float(r.W), float(r.h)};

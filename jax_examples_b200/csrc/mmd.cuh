@@ -122,7 +122,9 @@ struct __align__(16) Task {
 static_assert(sizeof(Task) == 16, "tasks are read as one vector");
 
 constexpr double kTwoPi25 = 34.986836655249725693;  // 2 pi^{5/2}
-constexpr double kSqrt8Pi25 = 11.8299343455912257556;    // sqrt(8 pi^{5/2})
+// sqrt(8 pi^{5/2}) in two parts: the first alone is 6.1e-17 off, which both
+// sides of a quartet share (1.2e-16 in every integral, always the same way).
+constexpr double kSqrt8Pi25 = 11.8299343455912257556, kSqrt8Pi25Lo = -7.1877868215575968e-16;
 
 // ---------------------------------------------------------------- E coeffs
 
