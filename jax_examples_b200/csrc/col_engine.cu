@@ -180,13 +180,11 @@ template <typename T, int LA, int LB, int LC, int LD>
 static cudaError_t launch_col_jk_class(const JKParams& p, cudaStream_t s) {
   if (p.n_tasks == 0) return cudaSuccess;
   const size_t sm = kColWarps * sizeof(ColSmem<T, LA, LB, LC, LD>) + 4 * kColSumWords;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(col_jk_kernel<T, LA, LB, LC, LD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  // on every launch: the limit is the current device's, and contexts of several
+  // devices and threads come here
+  cudaError_t e = cudaFuncSetAttribute(col_jk_kernel<T, LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sm);
+  if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)((p.n_tasks + kColWarps - 1) / kColWarps);
   col_jk_kernel<T, LA, LB, LC, LD><<<grid, 32 * kColWarps, sm, s>>>(p);
   return cudaGetLastError();

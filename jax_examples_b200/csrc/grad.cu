@@ -380,14 +380,10 @@ cudaError_t launch_warp_grad(int la, int lb, int lc, int ld, const GradParams& p
   if (p.n_tasks == 0) return cudaSuccess;
   const GradLayout ly(la, lb, lc, ld);
   const size_t sm = (size_t)kGradWarps * ly.total * sizeof(double);
-  static size_t configured = 0;
-  if (sm > configured) {
-    // the largest class, (dd|dd), needs 4 x 36 KB
-    cudaError_t e = cudaFuncSetAttribute(warp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kGradWarps * GradLayout(2, 2, 2, 2).total * sizeof(double)));
-    if (e != cudaSuccess) return e;
-    configured = (size_t)kGradWarps * GradLayout(2, 2, 2, 2).total * sizeof(double);
-  }
+  // the current device's limit, for the largest class: (dd|dd) needs 4 x 36 KB
+  cudaError_t e = cudaFuncSetAttribute(warp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(kGradWarps * GradLayout(2, 2, 2, 2).total * sizeof(double)));
+  if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)((p.n_tasks + kGradWarps - 1) / kGradWarps);
   warp_grad_kernel<<<grid, 32 * kGradWarps, sm, s>>>(p, la, lb, lc, ld);
   return cudaGetLastError();

@@ -398,13 +398,9 @@ template <int LA, int LB, int LC, int LD>
 static cudaError_t launch_grad_row_class(const GradParams& p, cudaStream_t s) {
   if (p.n_tasks == 0) return cudaSuccess;
   const size_t sm = kGRowWarps * sizeof(GRowSmem<LA, LB, LC, LD>);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e =
-        cudaFuncSetAttribute(grad_row_kernel<LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  cudaError_t e =  // the current device's limit, see launch_col_jk_class
+      cudaFuncSetAttribute(grad_row_kernel<LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)((p.n_tasks + kGRowWarps - 1) / kGRowWarps);
   grad_row_kernel<LA, LB, LC, LD><<<grid, 32 * kGRowWarps, sm, s>>>(p);
   return cudaGetLastError();
