@@ -254,11 +254,13 @@ int jqc_get_grad_engine(jqc_ctx *ctx, int *engines21);
 /* Autotuner: times every class of the J/K build for this density, precision
  * and screening (classes serialised, CUDA events, best of two, or one when a
  * build takes over 30 ms) over the engines, then threads (128, 256) x
- * persistent, then lane_prims (64, 128, 256, 512), keeps the fastest
+ * persistent, then lane_prims (64, 128, 256, 512; 256 stays where a short
+ * list makes them the same), keeps the fastest
  * shape per class and rebuilds the work list with it.  With cache_path, a
  * line "signature<TAB>84 integers" is appended; a later call whose signature
- * (device, settings, order of magnitude of each class's quartet count)
- * matches a line applies it without timing and sets *from_cache = 1.
+ * (version, device, settings, accumulator copies, order of magnitude of each
+ * class's quartet count) matches a line applies it without timing and sets
+ * *from_cache = 1.
  * J and K are overwritten.  Synchronizes.  No reference counterpart. */
 int jqc_autotune(jqc_ctx *ctx, int n_dens, const double *D, double *J, double *K, int precision_mode,
                  double mixed_tau, double dens_tau, const char *cache_path, int *from_cache, void *stream);

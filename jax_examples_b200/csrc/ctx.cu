@@ -876,6 +876,12 @@ static int jk_copies(int n, int n_dens) {
   return r;
 }
 static size_t jk_acc_size(int n, int n_dens) { return (size_t)jk_copies(n, n_dens) * 2 * n_dens * n * n; }
+// Without room for the copies a build adds straight into J and K.
+static void reserve_jk_copies(jqc_ctx* c, int n_dens) {
+  if (jk_copies(c->n_bf, n_dens) > 1 &&
+      c->d_acc[n_dens - 1].reserve(jk_acc_size(c->n_bf, n_dens)) != cudaSuccess)
+    (void)cudaGetLastError();
+}
 
 // One J/K build over work list `ts`: zero J/K, density maxima (when dmax is
 // given), the class kernels on the side streams (forked from and joined back
@@ -1691,10 +1697,7 @@ static int jk_impl(jqc_ctx* c, int n_dens, const double* D, double* J, double* K
     dmax = c->d_dmax.ptr;
     dmax_top = dmax + (size_t)c->n_shell * c->n_shell;
   }
-  // Without room for the copies the build adds straight into J and K.
-  if (!capturing && jk_copies(c->n_bf, n_dens) > 1 &&
-      c->d_acc[n_dens - 1].reserve(jk_acc_size(c->n_bf, n_dens)) != cudaSuccess)
-    (void)cudaGetLastError();
+  if (!capturing) reserve_jk_copies(c, n_dens);
   return run_jk_set(c, c->jk_cur, n_dens, D, J, K, dmax, dmax_top, dens_tau, s, class_ms);
 }
 
@@ -1805,11 +1808,12 @@ int jqc_get_grad_engine(jqc_ctx* c, int* engines21) {
   return JQC_OK;
 }
 
-// Workload signature for the tuning cache: device, precision settings and
+// Workload signature for the tuning cache: version of the work lists and
+// kernels that were timed, device, precision settings, accumulator copies and
 // the order of magnitude of the screened quartets of every class.
 static std::string tune_signature(jqc_ctx* c, const TaskSet* ts, int n_dens, int precision_mode, double dens_tau) {
   cudaDeviceProp prop;
-  std::string sig = "jqc-tune1";
+  std::string sig = "jqc-tune2";
   if (cudaGetDeviceProperties(&prop, c->device) == cudaSuccess) {
     std::string name = prop.name;
     for (char& ch : name)
@@ -1817,7 +1821,8 @@ static std::string tune_signature(jqc_ctx* c, const TaskSet* ts, int n_dens, int
     sig += " dev=" + name + "/" + std::to_string(prop.multiProcessorCount);
   }
   sig += " mode=" + std::to_string(precision_mode) + " ndens=" + std::to_string(n_dens) +
-         " dscreen=" + std::to_string(dens_tau > 0.0 ? 1 : 0) + " q=";
+         " dscreen=" + std::to_string(dens_tau > 0.0 ? 1 : 0) +
+         " copies=" + std::to_string(jk_copies(c->n_bf, n_dens)) + " q=";
   for (int prec = 0; prec < 2; ++prec)
     for (int qc = 0; qc < kNumQuartetClasses; ++qc) {
       const long long q = ts->class_quartets[prec][qc];
@@ -1886,6 +1891,7 @@ int jqc_autotune(jqc_ctx* c, int n_dens, const double* D, double* J, double* K, 
     dmax = c->d_dmax.ptr;
     dmax_top = dmax + (size_t)c->n_shell * c->n_shell;
   }
+  reserve_jk_copies(c, n_dens);  // the classes are timed as jqc_jk runs them
   // per-class time of the current settings: min over two timed builds, or
   // one when a build takes long enough (> 30 ms) for one to be steady
   double ms[2 * kNumQuartetClasses], best_ms[kNumQuartetClasses];
@@ -1950,13 +1956,20 @@ int jqc_autotune(jqc_ctx* c, int n_dens, const double* D, double* J, double* K, 
           best[qc].persistent = pe;
         }
     }
-  // 4. bra primitive chunk (work list rebuilt per value)
+  // 4. primitive quartets a lane (work list rebuilt per value).  Short lists take
+  // fewer than the value (lane_prim_limit): values that give the limit of one
+  // already timed would give its list again, and noise would choose.
   const int lp_opts[3] = {64, 128, 512};
+  const long long prims = c->jk_cur->n_prim_quartets;
+  std::vector<int> timed{lane_prim_limit(prims, kMaxLanePrims, c->sms, false)};
   for (int qc = 0; qc < kNumQuartetClasses; ++qc) {
     c->tune[qc].threads = best[qc].threads;
     c->tune[qc].persistent = best[qc].persistent;
   }
   for (int li = 0; li < 3; ++li) {
+    const int limit = lane_prim_limit(prims, lp_opts[li], c->sms, false);
+    if (std::find(timed.begin(), timed.end(), limit) != timed.end()) continue;
+    timed.push_back(limit);
     for (int qc = 0; qc < kNumQuartetClasses; ++qc) c->tune[qc].lane_prims = lp_opts[li];
     rc = rebuild();
     if (rc) return rc;
