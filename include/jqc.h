@@ -116,8 +116,9 @@ int jqc_set_molecule_activity(jqc_ctx *ctx, const int *d_active);
  * would use it: out[0] shell pairs, out[1] kept pairs, out[2] screened
  * canonical quartets on the FP64 path, out[3] on the FP32 path, out[4]
  * primitive quartets (both), out[5] Cartesian basis functions, out[6] warp
- * tasks, out[7] kernel launches per jqc_jk call.  No reference counterpart
- * (the reference never screens: integrals/screening.py is unused). */
+ * tasks, out[7] kernel launches of a jqc_jk call without density screening or
+ * molecule activity (those launch a few more).  No reference counterpart (the
+ * reference never screens: integrals/screening.py is unused). */
 int jqc_stats(jqc_ctx *ctx, int precision_mode, double mixed_tau, long long *out8);
 
 /* Per-class counters: for p in {FP64, FP32 path} and the 21 quartet classes

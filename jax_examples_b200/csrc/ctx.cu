@@ -989,8 +989,7 @@ static int run_jk_set(jqc_ctx* c, const TaskSet* ts, int n_dens, const double* D
   if (acc != nullptr) {
     JQC_CUDA_CHECK(launch_sum_symmetrize(acc, copies, J, K, n_dens, n, s));
   } else {
-    JQC_CUDA_CHECK(launch_symmetrize(J, n_dens, n, s));
-    JQC_CUDA_CHECK(launch_symmetrize(K, n_dens, n, s));
+    JQC_CUDA_CHECK(launch_symmetrize(J, K, n_dens, n, s));
   }
   return JQC_OK;
 }
@@ -1377,7 +1376,7 @@ int jqc_stats(jqc_ctx* c, int precision_mode, double mixed_tau, long long* out) 
   out[3] = c->jk_cur->n_quartets[1];
   out[4] = c->jk_cur->n_prim_quartets;
   out[5] = c->n_bf;
-  int launches = 2;  // J and K symmetrization
+  int launches = 1;  // J and K symmetrization, with or without accumulator copies
   for (int prec = 0; prec < 2; ++prec)
     for (int qc = 0; qc < kNumQuartetClasses; ++qc) launches += c->jk_cur->cnt[prec][qc] > 0;
   out[6] = (long long)c->jk_cur->n_tasks;

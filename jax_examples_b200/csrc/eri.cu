@@ -320,15 +320,15 @@ cudaError_t launch_compact(const CompactSeg* segs, const long long* seg_start, i
   return cudaGetLastError();
 }
 
-// M <- M + M^T for `count` consecutive n x n matrices.
-__global__ void symmetrize_kernel(double* M, int count, int n) {
+// M <- M + M^T for the `count` n x n matrices of J and of K.
+__global__ void symmetrize_kernel(double* __restrict__ J, double* __restrict__ K, int count, int n) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nn = (long long)n * n;
-  if (idx >= nn * count) return;
+  if (idx >= 2 * nn * count) return;
   const int m = int(idx / nn);
   const int i = int((idx % nn) / n), j = int(idx % n);
   if (i < j) return;
-  double* A = M + m * nn;
+  double* A = m < count ? J + m * nn : K + (m - count) * nn;
   if (i == j) {
     A[(size_t)i * n + i] *= 2.0;
   } else {
@@ -338,10 +338,10 @@ __global__ void symmetrize_kernel(double* M, int count, int n) {
   }
 }
 
-cudaError_t launch_symmetrize(double* M, int count, int n, cudaStream_t s) {
-  const long long tot = (long long)n * n * count;
+cudaError_t launch_symmetrize(double* J, double* K, int count, int n, cudaStream_t s) {
+  const long long tot = 2LL * n * n * count;
   if (tot == 0) return cudaSuccess;
-  symmetrize_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(M, count, n);
+  symmetrize_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(J, K, count, n);
   return cudaGetLastError();
 }
 

@@ -131,7 +131,8 @@ cudaError_t launch_boys(const double* T, long long n, int mmax, void* out, bool 
 // densities; with dmax_top non-null also the largest of them into *dmax_top.
 cudaError_t launch_dmax(const double* D, int n_dens, int n, int n_shell, const int* ao, const int* l, float* dmax,
                         float* dmax_top, cudaStream_t s);
-cudaError_t launch_symmetrize(double* M, int count, int n, cudaStream_t s);
+// J <- J + J^T and K <- K + K^T, count n x n matrices each.
+cudaError_t launch_symmetrize(double* J, double* K, int count, int n, cudaStream_t s);
 // The compact records (recf: may be null) of n_pairs shell pairs from their
 // primitive pairs.
 cudaError_t launch_prim_rec(const ShellPair* pairs, int n_pairs, const PrimPair* pp, PrimRec* rec, PrimRecF* recf,

@@ -73,3 +73,18 @@ def test_autotune_times_the_builds_that_follow(tmp_path):
     open(path, "w").write(text.replace("jqc-tune2", "jqc-tune1"))
     assert _autotune(eng, D, path) == 0
     eng.close()
+
+
+@pytest.mark.parametrize("copies", [True, False])
+@pytest.mark.parametrize("basis", ["sto-3g", "6-31g*"])
+def test_launch_count_of_the_statistics(basis, copies):
+    """launches_per_jk is the number of kernels in a captured build, with
+    accumulator copies and (two densities, captured before any build of two)
+    without them."""
+    eng = _engine(2, basis)
+    D = _densities(eng, 1 if copies else 2)
+    eng.jk(_densities(eng, 1))
+    kernels, memsets = _captured_nodes(eng, D)
+    assert memsets == (1 if copies else 2)
+    assert kernels == eng.stats("fp64")["launches_per_jk"]
+    eng.close()
