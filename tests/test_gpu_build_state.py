@@ -88,3 +88,36 @@ def test_launch_count_of_the_statistics(basis, copies):
     assert memsets == (1 if copies else 2)
     assert kernels == eng.stats("fp64")["launches_per_jk"]
     eng.close()
+
+
+def _tune(eng, lane_prims=None, engine=None):
+    cfg = np.zeros(84, dtype=np.int32)
+    _abi.call("jqc_get_tuning", eng._ctx, cfg.ctypes.data_as(_abi._ip))
+    if lane_prims is not None:
+        cfg.reshape(21, 4)[:, 1] = lane_prims
+    if engine is not None:
+        cfg.reshape(21, 4)[:, 3] = engine
+    _abi.call("jqc_set_tuning", eng._ctx, cfg.ctypes.data_as(_abi._ip))
+
+
+@pytest.mark.parametrize("waters,lane_prims", [(2, 5), (4, 5), (12, 5), (12, 256)])
+def test_lists_of_several_host_threads(waters, lane_prims):
+    """Lists of one, four and sixteen host threads, cut with remainders on both
+    sides of a quartet (5 of 9 and 36 primitive pairs), give the J/K of the
+    runtime-class engine, whose tasks have one ket each (same integrals in
+    another order: 1e-12 of the largest element)."""
+    eng = _engine(waters, "6-31g*", schwarz_tau=1e-10)
+    D = _densities(eng, 1)
+    _tune(eng, engine=2)
+    J0, K0 = eng.jk(D)
+    tasks = eng.stats("fp64")["tasks"]
+    eng.close()
+    eng = _engine(waters, "6-31g*", schwarz_tau=1e-10)
+    _tune(eng, lane_prims=lane_prims)
+    J, K = eng.jk(D)
+    st = eng.stats("fp64")
+    assert st["tasks"] != tasks
+    assert (st["kept_pairs"] >= 512) == (waters >= 4) and (st["kept_pairs"] >= 4096) == (waters >= 12)
+    for x, y in ((J, J0), (K, K0)):
+        assert float((x - y).abs().max()) < 1e-12 * float(y.abs().max())
+    eng.close()
