@@ -15,9 +15,11 @@
  *     in libint order (lx descending, then ly descending), as
  *     jax_qc/integrals/mcmurchie_davidson.py:39-50 and overlap.py:58-64.
  *   - A context's device scratch (density block maxima, the compacted work
- *     items of screened builds, gradient force slots) is shared by all calls
- *     on it: calls on one context must be ordered on the GPU (one stream, or
- *     streams ordered by events).  Different contexts are independent.
+ *     items of screened builds, the J/K accumulator copies, gradient force
+ *     slots) and its side streams are shared by all calls on it, unscreened
+ *     builds and graph replays included: calls on one context must be ordered
+ *     on the GPU (one stream, or streams ordered by events).  Different
+ *     contexts are independent.
  */
 #ifndef JQC_H_
 #define JQC_H_
@@ -233,12 +235,14 @@ int jqc_graph_destroy(jqc_ctx *ctx, int graph_id);
 
 /* Launch shape of each of the 21 quartet classes, cfg[4q..4q+3] =
  * threads per block (64/128/256), lane_prims (at most that many primitive
- * quartets per lane and task: the bra primitive pairs of a quartet are split
- * into chunks accordingly), persistent (1: grid capped at the resident
- * blocks, warps stride over the task list) and engine (0: register kernels,
- * lane = ket shell pair, classes with L <= 6; 1: column engine, one warp per
- * quartet, lane = ket Cartesian pair, classes with L >= 5; 2: runtime-class
- * warp engine, every class).  threads and persistent apply to the register
+ * quartets per lane and task, fewer while the whole list is short: the bra
+ * primitive pairs of a quartet are split into chunks accordingly, and in the
+ * register kernels the ket's where one bra primitive is still too long),
+ * persistent (1: grid capped at the resident blocks, warps stride over the
+ * task list) and engine (0: register kernels, lane = ket shell pair, classes
+ * with L <= 6; 1: column engine, one warp per quartet, lane = bra Hermite
+ * index on the ket side and ket Cartesian pair on the bra side, classes with
+ * L >= 5; 2: runtime-class warp engine, every class).  threads and persistent apply to the register
  * kernels only.  A new lane_prims or a change to or from the register engine
  * rebuilds the work lists.  No reference counterpart. */
 int jqc_get_tuning(jqc_ctx *ctx, int *cfg84);

@@ -916,7 +916,7 @@ static TaskSet* find_jk_tasks(jqc_ctx* c, int mode, double mixed_tau) {
   return nullptr;
 }
 
-constexpr long long kShortListPrims = 20000000;  // see launch_order
+constexpr long long kShortListPrims = 20000000;  // on 148 multiprocessors, see launch_order
 // Side streams for a list's kernels: two kernels each, so that a small basis
 // (six classes) does not pay for events of streams it hardly uses.  Measured
 // with 4 / 6 / 8 / 12 streams, us: (H2O)3 UHF 367 / 346 / 337 / 346, (H2O)16 mixed

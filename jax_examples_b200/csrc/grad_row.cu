@@ -406,8 +406,9 @@ static cudaError_t launch_grad_row_class(const GradParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Gradient classes with a row-engine kernel: the two it is the fastest in, and
-// the L <= 4 ones where engine code 1 asks for it.
+// Gradient classes with a row-engine kernel: (dd|dp) and (dd|dd), where it is the
+// fastest, and the two of L <= 4 that engine code 1 has always named; no default
+// takes those, they are a second form to check the register kernels against.
 #define JQC_FOR_GRAD_ROW_CLASSES(X) \
   X(11, 2, 1, 1, 0)                 \
   X(15, 2, 2, 0, 0)                 \

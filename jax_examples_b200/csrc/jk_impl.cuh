@@ -299,17 +299,25 @@ struct JKBody {
   }
 };
 
-// Warps walk the task list with a grid stride: one task per warp when the
-// grid covers the list, several (a persistent grid of resident blocks) when
-// the launch caps the grid.
 // Registers a thread may use.  The FP64 classes of low L wait on loads and on
 // FP64 results, and a few more resident warps are worth a few spilled values;
 // the larger ones lose more to the spills.  (H2O)16 full build, each class by
-// itself, us: (ps|ss) 98 -> 80 registers 942 -> 860 (72: 862, 96: 857, 128:
-// 905), (pp|ss) 138 -> 128 243 -> 225 (96: 235, 168: 246), (ds|ps) 180 -> 168
-// 614 -> 532 (96: 661, 128: 538), (dp|ss) 210 -> 128 385 -> 320 (96: 386, 168:
-// 337); every other class was slowest at the ends of 64 .. 168 and fastest at
-// the value here or unrestricted, and the FP32 classes did not care.
+// itself, us:
+//   registers  64   80   96  128  168  255
+//   (ss|ss)   533  517  547  606  591  588
+//   (ps|ss)   880  843  854  909  895  891
+//   (ps|ps)   450  386  374  372  418  416
+//   (pp|ss)   310  231  214  216  238  237
+//   (pp|ps)   935  581  425  270  236  254
+//   (ds|ss)   538  470  452  485  526  526
+//   (ds|ps)  1048  776  635  516  526  581
+//   (dp|ss)   572  422  358  295  302  361
+//   (dp|ps)  1169  720  585  497  442  472
+// and the other classes are fastest unrestricted.  (ds|ps) has 168 (532 against 538
+// at 128 when the caps were chosen); (ds|ss) at 96, (pp|ps) and (dp|ps) at 168 are
+// measured here but not taken.  FP32, every quartet of the same build: (ss|ss)
+// 340 at 64, 330 from 96 up; (ps|ss) 522 / 580 / 643 at 64 / 80 / 96; the others'
+// caps are not tuned ((ds|ss) 352 at 64, 459 unrestricted).
 template <typename T>
 __host__ __device__ constexpr int jk_register_cap(int la, int lb, int lc, int ld) {
   const int qc = quartet_class(pair_class(la, lb), pair_class(lc, ld));
@@ -317,6 +325,9 @@ __host__ __device__ constexpr int jk_register_cap(int la, int lb, int lc, int ld
   return qc <= 1 ? 80 : (qc == 2 || qc == 3 || qc == 6 || qc == 10) ? 128 : qc == 7 ? 168 : 255;
 }
 
+// Warps walk the task list with a grid stride: one task per warp when the
+// grid covers the list, several (a persistent grid of resident blocks) when
+// the launch caps the grid.
 template <typename T, int LA, int LB, int LC, int LD>
 __global__ void __maxnreg__(jk_register_cap<T>(LA, LB, LC, LD)) jk_kernel(const JKParams prm) {
   constexpr int NS = class_split(LA, LB, LC, LD);

@@ -112,6 +112,29 @@ def test_launch_count_of_the_statistics(basis, copies):
     eng.close()
 
 
+@pytest.mark.parametrize("dens_tau", [0.0, 1e-9])
+def test_captured_gradient_on_the_side_streams(dens_tau):
+    """A gradient captured into a graph forks to the side streams and back: replays
+    follow the density in the captured buffer and agree with calls (1e-12 of the
+    largest component)."""
+    eng = _engine(3, "6-31g*")
+    D = _densities(eng, 1)
+    g0 = grad_two_electron(eng, list(D), 1.0, 0.5, dens_tau=dens_tau)
+    out = torch.zeros_like(g0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        _abi.call("jqc_grad2e_ex", eng._ctx, 1, _ptr(D), 1.0, 0.5, dens_tau, _ptr(out),
+                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), None)
+    for seed in (0, 7):
+        D.copy_(_densities(eng, 1, seed))
+        ref = grad_two_electron(eng, list(D), 1.0, 0.5, dens_tau=dens_tau)
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert float((out - ref).abs().max()) < 1e-12 * max(1.0, float(ref.abs().max()))
+    eng.close()
+
+
 def _tune(eng, lane_prims=None, engine=None):
     cfg = np.zeros(84, dtype=np.int32)
     _abi.call("jqc_get_tuning", eng._ctx, cfg.ctypes.data_as(_abi._ip))
