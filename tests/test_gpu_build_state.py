@@ -10,7 +10,6 @@ from types import SimpleNamespace
 import numpy as np
 import pytest
 import torch
-from cuda.bindings import runtime as rt
 
 from jax_examples_b200 import DirectERI, _abi
 from jax_examples_b200 import basis as pb
@@ -48,6 +47,7 @@ def _capture(eng, D):
 
 def _captured_nodes(eng, D):
     """(kernels, memsets) of a build captured into a graph."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
     g, _, _ = _capture(eng, D)
     raw = rt.cudaGraph_t(g.raw_cuda_graph())
     err, _, count = rt.cudaGraphGetNodes(raw)
@@ -59,6 +59,7 @@ def _captured_nodes(eng, D):
 
 def _zeroed_bytes(eng, D):
     """Bytes that a captured build sets to zero first."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
     g, _, _ = _capture(eng, D)
     raw = rt.cudaGraph_t(g.raw_cuda_graph())
     _, _, count = rt.cudaGraphGetNodes(raw)
